@@ -345,23 +345,12 @@ def time_device(corr, sd_dev, dres, stream, steps, warmup, local, dist=None, clo
 # (workload, kernel): C3 captured at a 16 ms subint (250 blocks x 64
 # stations).  Traffic grows with the blocks a launch processes, so a step's
 # traffic is this figure times its blocks.
-F_DRAM_BYTES_PER_BLOCK = {("bench_c3", "fstep_sb_kernel"): (1.047047e9 + 4.136257e9) / 250}
+F_DRAM_BYTES_PER_BLOCK = {}
 
 
 def f_kernel_name(spec: JobSpec) -> str:
-    """The F-step kernel the library runs for this job (the station-block
-    kernel's domain: 512- to 8192-point transforms, whole-byte time samples of
-    1, 2, 4 or 8 bytes (real) or 4, 8 or 16 bytes (complex), payloads of whole
-    16-byte pieces, linear fringe rotation, plain VDIF)."""
-    F = spec.fftchannels
-    bpts_bits = spec.bits_per_timesample
-    bpts = bpts_bits // 8
-    ok = (512 <= F <= 8192 and bpts_bits % 8 == 0 and
-          (bpts in (4, 8, 16) if spec.is_complex else bpts in (1, 2, 4, 8)) and
-          spec.nbits * (2 if spec.is_complex else 1) in (1, 2, 4, 8, 16) and (spec.payload_bytes % 16 == 0))
-    if ok:
-        return "fstep_sb_kernel"
-    return "fstep_r16_kernel" if F >= 512 else "fstep_warp_kernel"
+    """The F-step kernel the library runs for this job."""
+    return "fstep_pair_kernel" if 128 <= spec.fftchannels <= 8192 else "fstep_cta_kernel"
 
 
 def roofline(spec: JobSpec, xstep: str, stage, peaks):

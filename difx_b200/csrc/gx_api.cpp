@@ -190,6 +190,8 @@ static gx_status setup(gx_handle *h)
   J.sampletime = 1.0 / (2.0 * f0.bw_mhz);
   if (cplx) J.sampletime *= 2.0;
   J.bw = f0.bw_mhz;
+  J.inv_fftlen = 1.0 / J.fftlen;
+  J.inv_nchan = 1.0 / J.nchan;
   J.nfreqs = h->nfmain;
   {
     double ffttime = 1000.0 * f0.nchan / f0.bw_mhz;
@@ -226,6 +228,7 @@ static gx_status setup(gx_handle *h)
   h->band_input.assign(d.nstations, std::vector<int>(s0.nbands, -1));
   h->maxnrf = 1;
   std::vector<DevStation> dst(d.nstations);
+  J.pair_same = 1;
   for (int s = 0; s < d.nstations; s++) {
     const gx_station_desc &x = d.stations[s];
     DevStation &D = dst[s];
@@ -252,6 +255,8 @@ static gx_status setup(gx_handle *h)
     }
     for (int b = 0; b < x.nbands; b++) D.band_polb[b] = (D.deltapol && x.band_pol[b] != 'R') ? 1 : 0;
     if (D.deltapol) J.deltapol_any = 1;
+    for (int b = 0; b + 1 < x.nbands; b += 2)
+      if (D.band_localfreq[b] != D.band_localfreq[b + 1] || D.band_polb[b] != D.band_polb[b + 1]) J.pair_same = 0;
   }
   // INTERLACEDVDIF stations: one weight row per band after the station rows
   h->interlaced_any = false;
@@ -992,8 +997,9 @@ static gx_status setup(gx_handle *h)
     }
     h->zacc_slice = h->zfreq.size() * (size_t)zx.npairs * zx.ST * zx.ST * h->nzchan;
   }
-  // F-step concurrency: FFT slots per CTA
-  {
+  // F-step concurrency: FFT slots per CTA of the slot-per-band kernel
+  h->nslots = 1;
+  if (!fstep_pair_eligible(J)) {
     int ns = std::min(J.nbands, 32);
     while (ns > 1 && (fstep_smem_bytes(J, h->maxnrf, ns) > 200 * 1024 || kFThreads % ns)) ns--;
     h->nslots = ns;
@@ -1161,12 +1167,12 @@ static gx_status setup(gx_handle *h)
       CKR(h, h->dalloc(&h->d_pcalrot, sizeof(float2) * h->pcal_rot.size()));
       CKR(h, cudaMemcpy(h->d_pcalrot, h->pcal_rot.data(), sizeof(float2) * h->pcal_rot.size(), cudaMemcpyHostToDevice));
     }
-    // The station-block F-step forms the bin sums itself when each thread's
+    // The paired-band F-step forms the bin sums itself when each thread's
     // samples share a bin (nbins divides F / 16); it then needs one slot of
     // partial sums per CTA group of the longest pass.
     h->pcal_fuse_bins = 0;
-    if (h->pcal_per_station && fstep_sb_eligible(J, false)) {
-      const int NT = J.fftlen / 16, G = (NT >= 256 ? NT : 256) / NT, nbins = h->pcal[0].nbins;
+    if (h->pcal_per_station && fstep_pair_eligible(J)) {
+      const int NT = J.fftlen / 16, G = fstep_pair_groups(J), nbins = h->pcal[0].nbins;
       if (nbins <= NT && NT % nbins == 0) {
         const int bpc = (J.sb_items > 0 ? J.sb_items : 4) * G;
         const long long slots = (long long)((h->chunk + bpc - 1) / bpc) * G;

@@ -48,13 +48,15 @@ struct DevJob {
   int ninputs;            // NI: padded spectra rows per freq
   int nfreqs;
   int blocks_per_send;
-  int sb_items;           // station-block F-step: FFT blocks per group and CTA (0: 4)
+  int sb_items;           // paired-band F-step: FFT blocks per group and CTA (0: 4)
   int flaglen;
   int lgstride;           // log2(stride): FFT length, channels and stride are powers of two
   int fringe_order;       // FRINGE ROTN ORDER: 1 pre-F linear, 2 pre-F quadratic, 0 post-F (real data)
   int deltapol_any;       // some station has a second (polarisation B) fractional-sample rotator
+  int pair_same;          // bands 2p and 2p + 1 share local freq and fractional-sample rotator at every station
   double sampletime;      // us
   double bw;              // MHz
+  double inv_fftlen, inv_nchan;   // 1 / fftlen, 1 / nchan (powers of two: exact)
   const float2 *twiddle;  // exp(-2 pi i m / F), m in [0, F), then the pass rows of r16::tw_pass_offset
   float lut[256];         // level of each sample code (VDIF decode table), staged to shared memory
   double lut_offset, lut_div;   // 8-bit codes: level = (code - lut_offset) / lut_div
@@ -120,7 +122,7 @@ struct PcalBand {
   long long rot0;
 };
 
-// Phase-cal bin sums formed inside the station-block F-step (the block's
+// Phase-cal bin sums formed inside the paired-band F-step (the block's
 // samples are decoded there anyway) instead of by a second read of the VDIF.
 // Taken when every station with phase-cal has one implicit-shift band per
 // recorded band, all with nbins bins, and nbins divides the transform's

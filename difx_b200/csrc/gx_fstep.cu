@@ -7,16 +7,11 @@
 //   blockparams_kernel  one thread per (station, block): FP64 delay, nearest
 //                       sample, fractional-sample error, linear interpolation
 //                       coefficients, frame-validity mask and data weight.
-//   fstep_r16_kernel    (FFT length 512-8192) a group of F / 16 threads per
-//                       (block, band), 16 samples per thread in registers,
-//                       radix-16 passes with padded shared-memory exchanges.
-//   fstep_warp_kernel   (FFT length 128-256) one warp per (block, band): the
-//                       warp builds its rotator tables, decodes and rotates
-//                       its samples into warp-private shared memory, runs the
-//                       FFT with warp-level synchronisation only and writes
-//                       the corrected spectrum row.
-//   fstep_cta_kernel    (longer FFTs not covered above) the bands of a block
-//                       are transformed concurrently in slots of one CTA.
+//   fstep_pair_kernel   (gx_fstep_pair.cuh; FFT lengths 128-8192, linear or
+//                       post-F fringe rotation) a group of F / 16 threads per
+//                       (station, block), two bands at a time.
+//   fstep_cta_kernel    (other lengths, quadratic rotation) the bands of a
+//                       block are transformed concurrently in slots of one CTA.
 //
 // Reference semantics followed (mpifxcorr/src):
 //   block validity / delay / nearest sample      mode.cpp:656-701
@@ -35,7 +30,7 @@
 #include <utility>
 #include "gx_dev.h"
 #include "gx_fcommon.cuh"
-#include "gx_fft16.h"
+#include "gx_xstep.h"
 
 namespace gx {
 
@@ -375,169 +370,7 @@ __device__ __forceinline__ float2 select_channel(const DevJob &J, const float2 *
 }
 
 // --------------------------------------------------------------------------
-// Warp-private FFT buffers are padded by one element every eight so that the
-// strided Stockham stores spread over the shared-memory banks.
-__device__ __forceinline__ int pidx(int i) { return i + (i >> 3); }
-
-// One compile-time Stockham pass (FL points, stride NS, radix R), in place in
-// one warp's buffer: every lane loads all of its butterflies' inputs, the warp
-// synchronises, then every lane stores its outputs.  Indices are shifts/masks.
-template <int FL, int NS, int R>
-__device__ __forceinline__ void warp_pass(float2 *buf, const float2 *tw, int lane)
-{
-  constexpr int NB = FL / R;
-  constexpr int PER = (NB + 31) / 32;
-  constexpr int TWSTEP = FL / (NS * R);
-  float2 v[PER][R];
-#pragma unroll
-  for (int p = 0; p < PER; p++) {
-    const int j = lane + 32 * p;
-    if (NB % 32 == 0 || j < NB) {
-      const int k = j & (NS - 1);
-#pragma unroll
-      for (int r = 0; r < R; r++) {
-        float2 x = buf[pidx(j + r * NB)];
-        if (r > 0 && NS > 1) x = cmul(x, tw[r * k * TWSTEP]);
-        v[p][r] = x;
-      }
-      if (R == 8) dft8(v[p]);
-      else if (R == 4) dft4(v[p][0], v[p][1], v[p][2], v[p][3]);
-      else {
-        float2 t = v[p][0];
-        v[p][0] = cadd(t, v[p][1]);
-        v[p][1] = csub(t, v[p][1]);
-      }
-    }
-  }
-  __syncwarp();
-#pragma unroll
-  for (int p = 0; p < PER; p++) {
-    const int j = lane + 32 * p;
-    if (NB % 32 == 0 || j < NB) {
-      const int k = j & (NS - 1);
-      const int idxD = (j - k) * R + k;   // (j / NS) * NS * R + k
-#pragma unroll
-      for (int r = 0; r < R; r++) buf[pidx(idxD + r * NS)] = v[p][r];
-    }
-  }
-  __syncwarp();
-}
-
-// All passes of an FL-point forward FFT in place: radix 8 while it fits, then 4 or 2.
-template <int FL, int NS>
-__device__ __forceinline__ void warp_fft(float2 *buf, const float2 *tw, int lane)
-{
-  if constexpr (NS < FL) {
-    constexpr int R = (NS * 8 <= FL) ? 8 : ((NS * 4 <= FL) ? 4 : 2);
-    warp_pass<FL, NS, R>(buf, tw, lane);
-    warp_fft<FL, NS * R>(buf, tw, lane);
-  }
-}
-
-// Warp-per-(block, band) F-step for FFT lengths up to 1024 (FL points,
-// complex sampling CPLX).
-constexpr int kWarpKernelThreads = 128;
-
-template <int FL, int CPLX>
-__global__ void __launch_bounds__(kWarpKernelThreads)
-fstep_warp_kernel(DevJob J, const DevStation *__restrict__ stations, SubintArrays S,
-                  const BlockParam *__restrict__ bp, int nblk, int blocks_per_cta, int wstride,
-                  float2 *__restrict__ spec)
-{
-  constexpr int NCH = CPLX ? FL : FL / 2;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ float s_lut[256];
-  __shared__ float2 s_tw[FL];
-  const int s = blockIdx.y;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-  const DevStation &st = stations[s];
-  const int Sd = J.stride, lgS = J.lgstride, nfr = J.nfr, half = J.half;
-  for (int i = tid; i < 256; i += blockDim.x) s_lut[i] = J.lut[i];
-  for (int i = tid; i < FL; i += blockDim.x) s_tw[i] = J.twiddle[i];
-  __syncthreads();
-
-  float2 *A = reinterpret_cast<float2 *>(smem_raw) + (size_t)warp * wstride;   // FL + FL/8 (padded)
-  float2 *rs = A + FL + FL / 8;   // S
-  float2 *rp = rs + Sd;        // nfr
-  float2 *fs = rp + nfr;       // S
-  float2 *fp = fs + Sd;        // half
-
-  const uint8_t *data = S.data[s];
-  const int fsamp = J.framesamples;
-  const int bits_ts = J.nbands * J.nbits * (CPLX ? 2 : 1);
-  const int cmask = (1 << J.nbits) - 1;
-  const int b0 = blockIdx.x * blocks_per_cta;
-  const int nbk = min(blocks_per_cta, nblk - b0);
-  const int nitems = nbk * J.nbands;
-  for (int it = warp; it < nitems; it += nwarps) {
-    const int bi = b0 + it / J.nbands;
-    const int bd = it % J.nbands;
-    const BlockParam P = band_param(bp, S, s, nblk, bi, J.nbands, bd);
-    const int lf = st.band_localfreq[bd];
-    const int f = st.freq_index[lf];
-    float2 *dst = spec + ((size_t)f * nblk + bi) * J.ninputs * NCH;
-    const int row = st.band_input[bd];
-    if (P.state == 0) {
-#pragma unroll
-      for (int c = lane; c < NCH; c += 32) dst[spec_offset(J, row, c)] = make_float2(0.f, 0.f);
-      continue;
-    }
-    const int ps = st.band_polb[bd] ? 1 : 0;
-    for (int e = lane; e < Sd + nfr; e += 32) {
-      const float2 v = fringe_entry(J, st, lf, e, P);
-      if (e < Sd) rs[e] = v;
-      else rp[e - Sd] = v;
-    }
-    for (int e = lane; e < Sd + half; e += 32) {
-      const float2 v = frac_entry(J, st, lf, ps, e, P);
-      if (e < Sd) fs[e] = v;
-      else fp[e - Sd] = v;
-    }
-    __syncwarp();
-    // decode + rotate: frame q and in-frame sample r advance incrementally
-    {
-      const int smp0 = P.nearestsample + lane;
-      int q = smp0 / fsamp;
-      int r = smp0 - q * fsamp;
-      q -= P.fr0;
-      const int bitband = bd * (CPLX ? 2 : 1) * J.nbits;
-#pragma unroll 4
-      for (int n = lane; n < FL; n += 32) {
-        float2 u = make_float2(0.f, 0.f);
-        if ((P.validmask >> q) & 1ull) {
-          const uint8_t *payload = data + ((long long)P.fr0 + q) * J.framebytes + 32;
-          const int bit0 = r * bits_ts + bitband;   // < 8 * payload bytes
-          u.x = s_lut[(__ldg(payload + (bit0 >> 3)) >> (bit0 & 7)) & cmask];
-          if (CPLX) {
-            const int bit1 = bit0 + J.nbits;
-            u.y = s_lut[(__ldg(payload + (bit1 >> 3)) >> (bit1 & 7)) & cmask];
-          }
-        }
-        const int k = n & (Sd - 1), j = n >> lgS;
-        const float2 rot = (j == 0) ? rs[k] : cmul_exact(rs[k], rp[j]);
-        A[pidx(n)] = CPLX ? cmul(rot, u) : make_float2(u.x * rot.x, u.x * rot.y);
-        r += 32;
-        while (r >= fsamp) { r -= fsamp; q++; }
-      }
-    }
-    __syncwarp();
-    warp_fft<FL, 1>(A, s_tw, lane);
-    const int lsb = st.lsb[lf];
-#pragma unroll 4
-    for (int c = lane; c < NCH; c += 32) {
-      float2 v;
-      if (!CPLX) v = A[pidx(lsb ? NCH + c : c)];
-      else if (!lsb) v = A[pidx(c)];
-      else if (c == 0) v = A[0];
-      else { v = A[pidx(FL - c)]; v.y = -v.y; }
-      dst[spec_offset(J, row, c)] = cmul(v, cmul_exact(fs[c & (Sd - 1)], fp[c >> lgS]));
-    }
-    __syncwarp();
-  }
-}
-
-// --------------------------------------------------------------------------
-// Slot-per-band F-step for long FFTs: the bands of a block in waves of
+// Slot-per-band F-step: the bands of a block in waves of
 // nslots concurrent FFTs, each over kFThreads / nslots threads.
 __global__ void __launch_bounds__(kFThreads)
 fstep_cta_kernel(DevJob J, const DevStation *__restrict__ stations, SubintArrays S,
@@ -583,7 +416,7 @@ fstep_cta_kernel(DevJob J, const DevStation *__restrict__ stations, SubintArrays
     const int nfe = Sd + nfr + (quad ? Sd : 0);
     for (int idx = tid; idx < nrf * nfe; idx += blockDim.x) {
       const int fi = idx / nfe, e = idx % nfe;
-      const float2 v = fringe_entry(J, st, fi, e, P);
+      const float2 v = fringe_entry(J, st, fi, e, P, J.stride, J.nfr);
       if (e < Sd) rsub[fi * Sd + e] = v;
       else if (e < Sd + nfr) rstep[fi * nfr + e - Sd] = v;
       else rquad[fi * Sd + e - Sd - nfr] = v;
@@ -593,7 +426,7 @@ fstep_cta_kernel(DevJob J, const DevStation *__restrict__ stations, SubintArrays
       const int ps = idx / (nrf * (Sd + half));
       const int r = idx % (nrf * (Sd + half));
       const int fi = r / (Sd + half), e = r % (Sd + half);
-      const float2 v = frac_entry(J, st, fi, ps, e, P);
+      const float2 v = frac_entry(J, st, fi, ps, e, P, J.stride, J.half);
       if (e < Sd) fsub[(ps * nrf + fi) * Sd + e] = v;
       else fstep[(ps * nrf + fi) * half + (e - Sd)] = v;
     }
@@ -665,277 +498,8 @@ fstep_cta_kernel(DevJob J, const DevStation *__restrict__ stations, SubintArrays
   }
 }
 
-// --------------------------------------------------------------------------
-// Register-resident F-step for long transforms: a group of NT = F / 16 threads
-// per (block, band) item, 16 samples per thread (x[j + NT t]) decoded and
-// fringe-rotated straight into registers, transformed by the radix-16 passes of
-// gx_fft16.h with padded shared-memory exchanges, and written from registers
-// after the sideband selection and fractional-sample correction.  A CTA holds
-// G = CTA / NT groups; groups synchronise on their own named barrier.
-#ifndef GX_R16_MINB
-#define GX_R16_MINB 4
-#endif
-template <int F>
-struct R16Launch {
-  static constexpr int NT = F / 16;
-  static constexpr int CTA = NT >= 256 ? NT : 256;
-  static constexpr int G = CTA / NT;
-  static constexpr int MINB = GX_R16_MINB * 256 / CTA;   // resident CTAs per SM the registers are sized for
-};
-
-
-// Samples x[j + NT t] (t = 0..15) of band bd of the block described by P,
-// decoded and fringe-rotated (mode.cpp:1160-1183): frame q and in-frame
-// sample r advance incrementally; all 16 raw loads are issued before use.
-// When a time sample of all bands is whole bytes and a step of NT samples
-// crosses at most one frame boundary (NT <= samples per frame), the byte
-// offset advances by a constant with one predicated correction per boundary;
-// otherwise each sample's bit offset is formed from (q, r).
-template <int F, int CPLX>
-__device__ __forceinline__ void r16_decode_rotate(const DevJob &J, const uint8_t *__restrict__ data,
-                                                  const BlockParam &P, int bd, int j, const float2 *rs,
-                                                  const float2 *rp, const float *s_lut, float2 (&v)[16])
-{
-  constexpr int NT = F / 16;
-  const int fsamp = J.framesamples;
-  const int bits_ts = J.nbands * J.nbits * (CPLX ? 2 : 1);
-  const int cmask = (1 << J.nbits) - 1;
-  const bool byte_pairs = CPLX && J.nbits == 8;   // (re, im) = one 16-bit word
-  const int smp0 = P.nearestsample + j;
-  int q = smp0 / fsamp;
-  int r = smp0 - q * fsamp;
-  q -= P.fr0;
-  const int bitband = bd * (CPLX ? 2 : 1) * J.nbits;
-  unsigned int raw[16];
-  if ((bits_ts & 7) == 0 && NT <= fsamp && (byte_pairs || !CPLX)) {
-    const int bpts = bits_ts >> 3, sh = bitband & 7;
-    const uint8_t *fr = data + ((long long)P.fr0 + q) * J.framebytes + 32 + (bitband >> 3);
-    int off = r * bpts;
-    bool ok = (P.validmask >> q) & 1ull;
-#pragma unroll
-    for (int t = 0; t < 16; t++) {
-      if (byte_pairs)
-        raw[t] = ok ? (unsigned int)__ldg(reinterpret_cast<const unsigned short *>(fr + off)) : 0xFFFFFFFFu;
-      else
-        raw[t] = ok ? ((unsigned int)(__ldg(fr + off) >> sh) & cmask) : 0xFFFFFFFFu;
-      r += NT;
-      off += NT * bpts;
-      if (r >= fsamp) {   // next frame: skip its header
-        r -= fsamp;
-        off -= fsamp * bpts;
-        q++;
-        fr += J.framebytes;
-        ok = (P.validmask >> q) & 1ull;
-      }
-    }
-  } else {
-#pragma unroll
-    for (int t = 0; t < 16; t++) {
-      raw[t] = 0xFFFFFFFFu;   // invalid frame: decodes to zero
-      if ((P.validmask >> q) & 1ull) {
-        const uint8_t *payload = data + ((long long)P.fr0 + q) * J.framebytes + 32;
-        const int bit0 = r * bits_ts + bitband;   // < 8 * payload bytes
-        if (byte_pairs) {
-          raw[t] = __ldg(reinterpret_cast<const unsigned short *>(payload + (bit0 >> 3)));
-        } else {
-          unsigned int w = (__ldg(payload + (bit0 >> 3)) >> (bit0 & 7)) & cmask;
-          if (CPLX) {
-            const int bit1 = bit0 + J.nbits;
-            w |= ((__ldg(payload + (bit1 >> 3)) >> (bit1 & 7)) & cmask) << 8;
-          }
-          raw[t] = w;
-        }
-      }
-      r += NT;
-      while (r >= fsamp) { r -= fsamp; q++; }
-    }
-  }
-  // rotator x[n] = sub[n mod S] * step[n / S]; with S dividing NT the sub entry
-  // is the same for all 16 samples of the thread
-  const int Sd = J.stride, lgS = J.lgstride;
-  const bool kfix = (NT & (Sd - 1)) == 0;
-  const float2 rsk = rs[j & (Sd - 1)];
-  const int jj0 = j >> lgS, jstep = NT >> lgS;
-#pragma unroll
-  for (int t = 0; t < 16; t++) {
-    float2 u = make_float2(0.f, 0.f);
-    if (raw[t] != 0xFFFFFFFFu) {
-      u.x = s_lut[raw[t] & 255u];
-      if (CPLX) u.y = s_lut[(raw[t] >> 8) & 255u];
-    }
-    float2 rot;
-    if (kfix) {
-      const int jj = jj0 + jstep * t;
-      rot = (jj == 0) ? rsk : cmul_exact(rsk, rp[jj]);
-    } else {
-      const int n = j + NT * t;
-      const int k = n & (Sd - 1), jj = n >> lgS;
-      rot = (jj == 0) ? rs[k] : cmul_exact(rs[k], rp[jj]);
-    }
-    v[t] = CPLX ? cmul(rot, u) : make_float2(u.x * rot.x, u.x * rot.y);
-  }
-}
-
-// Forward FFT of the group's transform: radix-16 passes with exchanges through
-// the padded buffer sm, then the final radix; register t ends with bin j + NT t.
-template <int F, int CTA, typename TW>
-__device__ __forceinline__ void r16_fft(float2 (&v)[16], int j, int g, float2 *sm, TW tw)
-{
-  using Pl = r16::Plan<F>;
-  constexpr int NT = Pl::NT;
-  int Ns = 1;
-#pragma unroll
-  for (int pass = 0; pass < Pl::L; pass++) {
-    r16::pass16<F>(v, j, Ns, tw);
-    if (!(pass == Pl::L - 1 && Pl::R0 == 1)) {
-      group_sync<NT, CTA>(g);
-      r16::store16(v, j, Ns, sm);
-      group_sync<NT, CTA>(g);
-      r16::load16<F>(v, j, sm);
-    }
-    Ns *= 16;
-  }
-  if constexpr (Pl::R0 > 1) r16::final_pass<F, Pl::R0>(v, j, tw);
-}
-
-
-template <int F, int CPLX>
-__global__ void __launch_bounds__(R16Launch<F>::CTA, R16Launch<F>::MINB)
-fstep_r16_kernel(DevJob J, const DevStation *__restrict__ stations, SubintArrays S,
-                 const BlockParam *__restrict__ bp, int nblk, int blocks_per_cta, int tabstride,
-                 float2 *__restrict__ spec)
-{
-  using Pl = r16::Plan<F>;
-  constexpr int NT = Pl::NT, CTA = R16Launch<F>::CTA, G = R16Launch<F>::G;
-  constexpr int NCH = CPLX ? F : F / 2;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ float s_lut[256];
-  const int s = blockIdx.y;
-  const int tid = threadIdx.x, g = tid / NT, j = tid % NT;
-  const DevStation &st = stations[s];
-  const int Sd = J.stride, lgS = J.lgstride, nfr = J.nfr, half = J.half;
-  for (int i = tid; i < 256; i += CTA) s_lut[i] = J.lut[i];
-  __syncthreads();
-
-  float2 *sm = reinterpret_cast<float2 *>(smem_raw) + (size_t)g * (Pl::SMEM + tabstride);
-  float2 *rs = sm + Pl::SMEM;  // S
-  float2 *rp = rs + Sd;        // nfr
-  float2 *fs = rp + nfr;       // S
-  float2 *fp = fs + Sd;        // half
-  const float2 *__restrict__ twg = J.twiddle;
-  auto tw = [twg](int m) { return __ldg(&twg[m]); };
-
-  const uint8_t *data = S.data[s];
-  const int b0 = blockIdx.x * blocks_per_cta;
-  const int nbk = min(blocks_per_cta, nblk - b0);
-  const int nitems = nbk * J.nbands;
-  for (int it = g; it < nitems; it += G) {
-    const int bi = b0 + it / J.nbands;
-    const int bd = it % J.nbands;
-    const BlockParam P = band_param(bp, S, s, nblk, bi, J.nbands, bd);
-    const int lf = st.band_localfreq[bd];
-    const int f = st.freq_index[lf];
-    const int row = st.band_input[bd];
-    float2 *dst = spec + ((size_t)f * nblk + bi) * J.ninputs * NCH;
-    if (P.state == 0) {
-      for (int c = j; c < NCH; c += NT) dst[spec_offset(J, row, c)] = make_float2(0.f, 0.f);
-      continue;
-    }
-    const int ps = st.band_polb[bd] ? 1 : 0;
-    group_sync<NT, CTA>(g);   // the group's previous item is done with the tables and the exchange buffer
-    for (int e = j; e < Sd + nfr; e += NT) {
-      const float2 v = fringe_entry(J, st, lf, e, P);
-      if (e < Sd) rs[e] = v;
-      else rp[e - Sd] = v;
-    }
-    for (int e = j; e < Sd + half; e += NT) {
-      const float2 v = frac_entry(J, st, lf, ps, e, P);
-      if (e < Sd) fs[e] = v;
-      else fp[e - Sd] = v;
-    }
-    group_sync<NT, CTA>(g);
-
-    float2 v[16];
-    r16_decode_rotate<F, CPLX>(J, data, P, bd, j, rs, rp, s_lut, v);
-    r16_fft<F, CTA>(v, j, g, sm, tw);
-    // register t holds bin j + NT t: sideband selection and fractional-sample correction
-    // (with S dividing NT, channel c mod S is the same for all the thread's bins:
-    // j mod S, or -j mod S for complex lower sideband)
-    const int lsb = st.lsb[lf];
-    const bool kfix = (NT & (Sd - 1)) == 0;
-    const float2 fsk = fs[((CPLX && lsb) ? -j : j) & (Sd - 1)];
-    float2 *drow = dst + spec_offset(J, row, 0);
-    auto emit = [&](int c, float2 val) {
-      drow[c] = cmul(val, cmul_exact(kfix ? fsk : fs[c & (Sd - 1)], fp[c >> lgS]));
-    };
-    // one unrolled loop per sideband, so that every channel index is j plus a constant
-    if (lsb) {
-#pragma unroll
-      for (int t = 0; t < 16; t++) {
-        float2 val = v[t];
-        int c;
-        if (r16_channel<F, CPLX>(t, j, 1, val, c)) emit(c, val);
-      }
-    } else {
-#pragma unroll
-      for (int t = 0; t < 16; t++) {
-        float2 val = v[t];
-        int c;
-        if (r16_channel<F, CPLX>(t, j, 0, val, c)) emit(c, val);
-      }
-    }
-  }
-}
-
-// --------------------------------------------------------------------------
-// The warp and radix-16 kernels hold the fringe rotator as two tables
-// (sub[k] step[j]); the quadratic order needs the full table of the CTA kernel.
-static bool use_warp_kernel(const DevJob &J) { return J.fftlen >= 128 && J.fftlen <= 1024 && J.fringe_order != 2; }
-
-static int warp_stride(const DevJob &J)
-{
-  int w = J.fftlen + J.fftlen / 8 + 2 * J.stride + J.nfr + (J.half > 0 ? J.half : 1);
-  return (w + 1) & ~1;   // keep each warp's region 16-byte aligned
-}
-
-// Register-resident radix-16 kernel for the transform lengths it is built for.
-static bool use_r16_kernel(const DevJob &J)
-{
-  const char *e = getenv("GX_FSTEP_R16_MIN");   // smallest length routed to it (tuning runs)
-  const int fmin = e ? atoi(e) : 512;
-  return J.fftlen >= fmin && J.fftlen >= 512 && J.fftlen <= 8192 && J.fringe_order != 2;
-}
-
-// Station-block kernel (gx_fstep_sb.cu) for the jobs it takes; GX_FSTEP_SB=0
-// selects the per-band kernels instead (comparison runs).
-bool fstep_sb_eligible(const DevJob &J, bool interlaced);
-cudaError_t fstep_sb_launch(const DevJob &J, const DevStation *stations, int maxnrf, int deltapol,
-                            const SubintArrays &S, int nblk, const BlockParam *bp, float2 *spec, cudaStream_t st,
-                            const PcalFuse *pf, bool *pcal_done);
-
-static bool use_sb_kernel(const DevJob &J, bool interlaced)
-{
-  const char *e = getenv("GX_FSTEP_SB");
-  if (e && atoi(e) == 0) return false;
-  return fstep_sb_eligible(J, interlaced);
-}
-
-static int r16_tabstride(const DevJob &J)
-{
-  return (2 * J.stride + J.nfr + (J.half > 0 ? J.half : 1) + 1) & ~1;
-}
-
-static int r16_groups(const DevJob &J)
-{
-  const int nt = J.fftlen / 16;
-  return nt >= 256 ? 1 : 256 / nt;
-}
-
 size_t fstep_smem_bytes(const DevJob &J, int nrf, int nslots)
 {
-  if (use_r16_kernel(J))
-    return (size_t)r16_groups(J) * (J.fftlen + J.fftlen / 16 + r16_tabstride(J)) * sizeof(float2);
-  if (use_warp_kernel(J)) return (size_t)(kWarpKernelThreads / 32) * warp_stride(J) * sizeof(float2);
   size_t b = (size_t)nslots * 2 * J.fftlen * sizeof(float2);
   b += (size_t)nrf * (J.stride + J.nfr) * sizeof(float2);
   b += (size_t)2 * nrf * (J.stride + (J.half > 0 ? J.half : 1)) * sizeof(float2);
@@ -1440,45 +1004,8 @@ cudaError_t fstep_launch(const DevJob &J, const DevStation *stations, int maxnrf
     dim3 grid((nblk + 7) / 8, J.nstations);
     edv4_kernel<<<grid, 256, 0, st>>>(J, stations, S, nblk, bp, weights);
   }
-  if (use_sb_kernel(J, S.bandmask != nullptr)) {
-    cudaError_t e = fstep_sb_launch(J, stations, maxnrf, J.deltapol_any, S, nblk, bp, spec, st, pf, pcal_done);
-    if (e != cudaErrorNotSupported) return e;
-    if (pcal_done) *pcal_done = false;
-  }
+  if (fstep_pair_eligible(J)) return fstep_pair_launch(J, stations, S, nblk, bp, spec, st, pf, pcal_done);
   const size_t sm = fstep_smem_bytes(J, maxnrf, nslots);
-  if (use_r16_kernel(J)) {
-    const int G = r16_groups(J);
-    // at least four items per group, so that groups overlap their barriers
-    const int bpc = std::max(1, (4 * G + J.nbands - 1) / J.nbands);
-    dim3 grid((nblk + bpc - 1) / bpc, J.nstations);
-    const int ts = r16_tabstride(J);
-#define GX_R16_CASE(FLV, CX)                                                                          \
-    if (J.fftlen == FLV && J.cplx == CX) {                                                            \
-      cudaError_t e = smem_opt_in((const void *)fstep_r16_kernel<FLV, CX>, sm);                       \
-      if (e != cudaSuccess) return e;                                                                 \
-      fstep_r16_kernel<FLV, CX><<<grid, R16Launch<FLV>::CTA, sm, st>>>(J, stations, S, bp, nblk, bpc, ts, spec); \
-      return cudaGetLastError();                                                                      \
-    }
-    GX_R16_CASE(512, 0) GX_R16_CASE(1024, 0) GX_R16_CASE(2048, 0) GX_R16_CASE(4096, 0) GX_R16_CASE(8192, 0)
-    GX_R16_CASE(512, 1) GX_R16_CASE(1024, 1) GX_R16_CASE(2048, 1) GX_R16_CASE(4096, 1) GX_R16_CASE(8192, 1)
-#undef GX_R16_CASE
-  }
-  if (use_warp_kernel(J)) {
-    // enough items per CTA that each warp has several (block, band) items
-    const int bpc = (J.nbands >= 8) ? 2 : 8;
-    dim3 grid((nblk + bpc - 1) / bpc, J.nstations);
-    const int ws = warp_stride(J);
-#define GX_WARP_CASE(FLV, CX)                                                                         \
-    if (J.fftlen == FLV && J.cplx == CX) {                                                            \
-      cudaError_t e = smem_opt_in((const void *)fstep_warp_kernel<FLV, CX>, sm);                      \
-      if (e != cudaSuccess) return e;                                                                 \
-      fstep_warp_kernel<FLV, CX><<<grid, kWarpKernelThreads, sm, st>>>(J, stations, S, bp, nblk, bpc, ws, spec); \
-      return cudaGetLastError();                                                                      \
-    }
-    GX_WARP_CASE(128, 0) GX_WARP_CASE(256, 0) GX_WARP_CASE(512, 0) GX_WARP_CASE(1024, 0)
-    GX_WARP_CASE(128, 1) GX_WARP_CASE(256, 1) GX_WARP_CASE(512, 1) GX_WARP_CASE(1024, 1)
-#undef GX_WARP_CASE
-  }
   {
     cudaError_t e = smem_opt_in((const void *)fstep_cta_kernel, sm);
     if (e != cudaSuccess) return e;

@@ -1,0 +1,13 @@
+// Station-pair F-step kernels (gx_fstep_pair.cuh) of complex data with phase-cal.
+#include "gx_fstep_pair.cuh"
+
+namespace gx {
+namespace pr {
+
+cudaError_t launch_cplx_pc(GX_PAIR_ARGS)
+{
+  return launch<1, true>(J, stations, S, nblk, items, D, bp, spec, pf, st);
+}
+
+}  // namespace pr
+}  // namespace gx

@@ -40,7 +40,7 @@ struct gx_handle {
   float2 *d_pcalrot = nullptr;
   float2 *d_pcalbins = nullptr;              // [chunk][pcal band][bin] partial bin sums
   int pcal_chunks = 0, pcal_maxbins = 0, pcal_per_station = 0;
-  // bin sums formed inside the station-block F-step (gx::PcalFuse): station
+  // bin sums formed inside the paired-band F-step (gx::PcalFuse): station
   // -> first phase-cal band (-1: none), on the device; 0 bins when not offered
   int *d_pcalfirst = nullptr;
   int pcal_fuse_bins = 0;

@@ -41,9 +41,13 @@ XmacShape xmac_shape(int NI);
 cudaError_t tma_map_f32_4d(CUtensorMap *map, const void *base, const cuuint64_t dims[4], const cuuint32_t box[4]);
 
 size_t fstep_smem_bytes(const DevJob &J, int nrf, int nslots);
-// Whether the station-block F-step (gx_fstep_sb.cu) takes this job.
-bool fstep_sb_eligible(const DevJob &J, bool interlaced);
-// F-step of one pass of blocks.  With pf, the station-block kernel also forms
+// The paired-band F-step (gx_fstep_pair.cuh): whether it takes this job, blocks
+// it has in flight per CTA, and its launch over one pass of blocks.
+bool fstep_pair_eligible(const DevJob &J);
+int fstep_pair_groups(const DevJob &J);
+cudaError_t fstep_pair_launch(const DevJob &J, const DevStation *stations, const SubintArrays &S, int nblk,
+                              const BlockParam *bp, float2 *spec, cudaStream_t st, const PcalFuse *pf, bool *pcal_done);
+// F-step of one pass of blocks.  With pf, the paired-band kernel also forms
 // the phase-cal bin sums when it takes the job; *pcal_done (if given) tells
 // whether it did (else the caller runs pcal_bins_launch).
 cudaError_t fstep_launch(const DevJob &J, const DevStation *stations, int maxnrf, const SubintArrays &S,
