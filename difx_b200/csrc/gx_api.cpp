@@ -272,6 +272,7 @@ static gx_status setup(gx_handle *h)
   }
   int ni = 0;
   for (int f = 0; f < d.nfreqs; f++) ni = count[f] > ni ? count[f] : ni;
+  J.nrows = ni;
   if (d.xstep < GX_XSTEP_FP32 || d.xstep > GX_XSTEP_AUTO) return h->fail(GX_ERR_ARG, "unknown xstep");
   h->xstep = d.xstep;
   if (d.xstep == GX_XSTEP_AUTO) {
@@ -932,7 +933,8 @@ static gx_status setup(gx_handle *h)
   } else {
     // Both X-steps move their accumulators through HBM once per pass (the
     // tensor-core form 128 x 128 complex per channel, the FP32 form its upper
-    // super-tiles), so passes are long: up to 40 GB of spectra, at most 30% of
+    // super-tiles) and every pass ends in a partly filled round of CTAs, so
+    // passes are long: up to 32768 blocks and 40 GB of spectra, at most 30% of
     // the device memory free at open.
     size_t spec_budget = size_t(40) << 30;
     {
@@ -940,7 +942,7 @@ static gx_status setup(gx_handle *h)
       if (h->device >= 0 && cudaSetDevice(h->device) == cudaSuccess && cudaMemGetInfo(&fr, &tot) == cudaSuccess)
         spec_budget = std::max(size_t(1) << 30, std::min(spec_budget, fr / 10 * 3));
     }
-    chunk = (int)std::min<size_t>(4096, std::max<size_t>(64, spec_budget / per_block));
+    chunk = (int)std::min<size_t>(32768, std::max<size_t>(64, spec_budget / per_block));
   }
   if (chunk > J.blocks_per_send) chunk = J.blocks_per_send;
   chunk = std::max(1, chunk);
@@ -970,7 +972,8 @@ static gx_status setup(gx_handle *h)
     long long base = (long long)((J.nchan + xs.CT - 1) / xs.CT) * xs.npairs * h->nfmain;
     // K-split: enough CTAs for at least two per SM, rounded to whole waves of
     // 148 SMs where possible, keeping at least 64 blocks per slice
-    const int kmax = std::max(1, std::min(16, chunk / 64));
+    // (up to 64 slices of 8 inputs, whose accumulators are small)
+    const int kmax = std::max(1, std::min(xs.ST == 8 ? 64 : 16, chunk / 64));
     int best = 1;
     double best_score = -1;
     for (int ks = 1; ks <= kmax; ks++) {
@@ -1174,9 +1177,12 @@ static gx_status setup(gx_handle *h)
     if (h->pcal_per_station && fstep_pair_eligible(J)) {
       const int NT = J.fftlen / 16, G = fstep_pair_groups(J), nbins = h->pcal[0].nbins;
       if (nbins <= NT && NT % nbins == 0) {
+        // a slot per group of a CTA of the longest pass at four blocks a group,
+        // at most 512 MB of sums (then a group takes more blocks)
         const int bpc = (J.sb_items > 0 ? J.sb_items : 4) * G;
-        const long long slots = (long long)((h->chunk + bpc - 1) / bpc) * G;
-        if (slots * (long long)h->pcal.size() * h->pcal_maxbins <= (64ll << 20)) {   // at most 512 MB of sums
+        const long long per_cta = (long long)G * (long long)h->pcal.size() * h->pcal_maxbins;
+        const long long slots = std::min<long long>((h->chunk + bpc - 1) / bpc, (64ll << 20) / per_cta) * G;
+        if (slots * 64 >= h->chunk) {
           std::vector<int> first(d.nstations, -1);
           for (size_t i = 0; i < h->pcal.size(); i += J.nbands) first[h->pcal[i].station] = (int)i;
           CKR(h, h->dalloc(&h->d_pcalfirst, sizeof(int) * first.size()));
@@ -1619,10 +1625,7 @@ gx_status gx_enqueue_subint(gx_handle *h, float2 *dev_results, cudaStream_t st)
   const int nbl = d.nbaselines;
   float4 *acc4 = reinterpret_cast<float4 *>(h->d_acc);
   auto mark = [&](int stage, bool start) -> gx_status { return timed ? record(h, st, stage, start) : GX_OK; };
-  // the tensor-core X-step stores its first chunk instead of adding to it
-  if (!h->tc) CKR(h, cudaMemsetAsync(h->d_acc, 0, sizeof(float2) * h->acc_slice * h->ks, st));
   const int nzr = (int)h->zrows.size(), nzf = (int)h->zfreq.size();
-  if (nzf) CKR(h, cudaMemsetAsync(h->d_accz, 0, sizeof(float2) * h->zacc_slice * h->zks, st));
   if (h->nbins > 0) {
     CKR(h, cudaMemsetAsync(h->d_accb, 0, sizeof(float2) * h->binents.size() * h->nbins * J.nchan, st));
     CKR(h, cudaMemsetAsync(h->d_wbins, 0, sizeof(float) * h->binitems.size() * h->nbins, st));
@@ -1637,7 +1640,8 @@ gx_status gx_enqueue_subint(gx_handle *h, float2 *dev_results, cudaStream_t st)
   // with channel averaging the finalise fills the full-resolution array first
   float2 *fin = h->avg > 1 ? h->d_full : dev_results;
   // one pass of nb blocks from block b0: F-step (and phase-cal bins), X-step, weights
-  auto pass = [&](int b0, int nb) -> gx_status {
+  // (first: the X-steps store their sums instead of adding to the accumulators)
+  auto pass = [&](int b0, int nb, bool first) -> gx_status {
     gx_status r;
     if ((r = mark(0, true)) != GX_OK) return r;
     const PcalFuse pf{h->d_pcalbins, h->d_pcalfirst, h->pcal_fuse_bins, h->pcal_maxbins, npc, h->pcal_chunks};
@@ -1654,9 +1658,10 @@ gx_status gx_enqueue_subint(gx_handle *h, float2 *dev_results, cudaStream_t st)
     if ((r = mark(1, true)) != GX_OK) return r;
     if (h->tc)
       CKR(h, xmac_tc_launch(h->d_spec, nb, J.nchan, h->nfmain, J.ninputs, h->ks, h->hilo, h->d_scale, acc4,
-                            b0 > 0 ? 1 : 0, h->d_err, st));
+                            first ? 0 : 1, h->d_err, st));
     else
-      CKR(h, xmac_fp32_launch(h->d_spec, nb, J.ninputs, J.nchan, h->nfmain, h->ks, h->d_acc, h->d_err, st, h->xvar));
+      CKR(h, xmac_fp32_launch(h->d_spec, nb, J.nrows, J.ninputs, J.nchan, h->nfmain, h->ks, h->d_acc, first ? 0 : 1, h->d_err,
+                              st, h->xvar));
     if (h->nbins > 0) {   // pulsar binning: the binned cross products and weights of this pass
       const double *avgphase = reinterpret_cast<const double *>(h->d_sub + h->o_avgphase);
       const double *dmoff = reinterpret_cast<const double *>(h->d_sub + h->o_dmoff);
@@ -1670,7 +1675,8 @@ gx_status gx_enqueue_subint(gx_handle *h, float2 *dev_results, cudaStream_t st)
     if (nzf) {   // zoom freqs: their rows of this pass's spectra, then their cross products
       CKR(h, zoom_gather_launch(h->d_zrows, nzr, h->d_spec, J.ninputs, J.nchan, h->d_specz, h->nzrows, h->nzchan, nb,
                                 st));
-      CKR(h, xmac_fp32_launch(h->d_specz, nb, h->nzrows, h->nzchan, nzf, h->zks, h->d_accz, h->d_err, st));
+      CKR(h, xmac_fp32_launch(h->d_specz, nb, h->nzrows, h->nzrows, h->nzchan, nzf, h->zks, h->d_accz, b0 > 0 ? 1 : 0, h->d_err,
+                              st));
       h->launches += 2;
     }
     CKR(h, weights_launch(h->d_w, nb, d.nstations, h->d_pairs, npairs, h->d_wacc, st));
@@ -1690,9 +1696,8 @@ gx_status gx_enqueue_subint(gx_handle *h, float2 *dev_results, cudaStream_t st)
     const double *uvd = reinterpret_cast<const double *>(h->d_sub + h->o_uvdelay);
     for (int iv = 0; iv * M < J.blocks_per_send; iv++) {
       const int i0 = iv * M, i1 = std::min(J.blocks_per_send, i0 + M);
-      if (iv > 0) CKR(h, cudaMemsetAsync(h->d_acc, 0, sizeof(float2) * h->acc_slice * h->ks, st));
       for (int b0 = i0; b0 < i1; b0 += h->chunk)
-        if ((r = pass(b0, std::min(h->chunk, i1 - b0))) != GX_OK) return r;
+        if ((r = pass(b0, std::min(h->chunk, i1 - b0), b0 == i0)) != GX_OK) return r;
       if ((r = mark(2, true)) != GX_OK) return r;
       CKR(h, uvshift_launch(h->d_uvents, (int)h->uvents.size(), h->d_acc, h->ks, h->acc_slice, J.nchan,
                             uvd + (size_t)iv * nbl * h->maxpc, nph, h->maxpc, h->d_uvfreqs, h->rsl, fin, st));
@@ -1701,7 +1706,7 @@ gx_status gx_enqueue_subint(gx_handle *h, float2 *dev_results, cudaStream_t st)
     }
   } else {
     for (int b0 = 0; b0 < J.blocks_per_send; b0 += h->chunk)
-      if ((r = pass(b0, std::min(h->chunk, J.blocks_per_send - b0))) != GX_OK) return r;
+      if ((r = pass(b0, std::min(h->chunk, J.blocks_per_send - b0), b0 == 0)) != GX_OK) return r;
   }
   if (h->kurt && (r = gx_kurtosis_end(h, st)) != GX_OK) return r;
   if ((r = mark(2, true)) != GX_OK) return r;

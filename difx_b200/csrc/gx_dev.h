@@ -46,6 +46,7 @@ struct DevJob {
   int half;               // numfracstrides / 2
   int unpacksamples;
   int ninputs;            // NI: padded spectra rows per freq
+  int nrows;              // rows in use of the fullest freq
   int nfreqs;
   int blocks_per_send;
   int sb_items;           // paired-band F-step: FFT blocks per group and CTA (0: 4)

@@ -67,7 +67,7 @@ static int pair_items(const DevJob &J, int nblk)
 
 // Whether the kernel can form the phase-cal sums of pf for this job and
 // launch: bins dividing the threads of a transform, one slot per group.
-bool fstep_pair_pcal_fits(const DevJob &J, const PcalFuse &pf, int nblk, int items)
+static bool fstep_pair_pcal_fits(const DevJob &J, const PcalFuse &pf, int nblk, int items)
 {
   const int NT = J.fftlen / 16, G = fstep_pair_groups(J);
   return pf.partial && pf.first && pf.nbins > 0 && pf.nbins <= NT && NT % pf.nbins == 0 &&
@@ -81,11 +81,12 @@ cudaError_t fstep_pair_launch(const DevJob &J, const DevStation *stations, const
   int items = pair_items(J, nblk);
   bool pc = false;
   if (pf) {
-    pc = fstep_pair_pcal_fits(J, *pf, nblk, items);
-    if (!pc && J.sb_items <= 0 && items < 4) {   // the slots are counted for four
-      pc = fstep_pair_pcal_fits(J, *pf, nblk, 4);
-      if (pc) items = 4;
-    }
+    // as many blocks per group as the slots need (the tuner's choice stands)
+    int most = items;
+    if (J.sb_items <= 0)
+      while (most < 64 && !fstep_pair_pcal_fits(J, *pf, nblk, most)) most++;
+    pc = fstep_pair_pcal_fits(J, *pf, nblk, most);
+    if (pc) items = most;
   }
   const PcalFuse pfv = pc ? *pf : PcalFuse{};
   if (pcal_done) *pcal_done = pc;

@@ -128,7 +128,7 @@ extern "C" gx_status gx_subint_device_noalloc(const gx_job_desc *desc, const gx_
   const size_t o_went = take(sizeof(WeightEntry) * (plan.wents.empty() ? 1 : plan.wents.size()));
   const size_t o_wacc = take(sizeof(float) * (nst + nbl));
   const size_t acc_slice = (size_t)J0.nfreqs * plan.xs.npairs * plan.xs.ST * plan.xs.ST * J0.nchan;
-  int ks = plan.ks;
+  int ks = std::min(plan.ks, 16);   // the scratch also holds the spectra
   const size_t per_block = sizeof(float2) * (size_t)J0.nfreqs * J0.ninputs * J0.nchan +
                            (sizeof(float) + sizeof(BlockParam)) * nst + 512;
   size_t fixed = off + align256(sizeof(float2) * acc_slice * ks);
@@ -228,7 +228,7 @@ extern "C" gx_status gx_subint_device_noalloc(const gx_job_desc *desc, const gx_
   for (int b0 = 0; b0 < J.blocks_per_send; b0 += chunk) {
     const int nb = std::min(chunk, J.blocks_per_send - b0);
     NA_CK(fstep_launch(J, d_st, plan.maxnrf, S, b0, nb, plan.nslots, d_spec, d_w, d_bp, st));
-    NA_CK(xmac_fp32_launch(d_spec, nb, J.ninputs, J.nchan, J.nfreqs, ks, d_acc, nullptr, st));
+    NA_CK(xmac_fp32_launch(d_spec, nb, J.nrows, J.ninputs, J.nchan, J.nfreqs, ks, d_acc, b0 > 0 ? 1 : 0, nullptr, st));
     NA_CK(weights_launch(d_w, nb, nst, d_pairs, nbl, d_wacc, st));
   }
   NA_CK(finalise_launch(d_prods, (int)plan.prods.size(), d_acc, ks, acc_slice, J.nchan, d_went,

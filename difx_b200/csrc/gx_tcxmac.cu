@@ -508,7 +508,8 @@ finalise_tc_kernel(const TcProdEntry *__restrict__ prods, const TcRowEntry *__re
 // 4-D FP32 tensor map over a dense row-major array (innermost dimension
 // first, strides implied by the dimensions), box `box`, no swizzle, no
 // interleave; out-of-bounds elements read as zeros.
-cudaError_t tma_map_f32_4d(CUtensorMap *map, const void *base, const cuuint64_t dims[4], const cuuint32_t box[4])
+cudaError_t tma_map_f32_4d(CUtensorMap *map, const void *base, const cuuint64_t dims[4], const cuuint32_t box[4],
+                           int pitch1)
 {
   static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
   if (!encode) {
@@ -519,7 +520,8 @@ cudaError_t tma_map_f32_4d(CUtensorMap *map, const void *base, const cuuint64_t 
     if (q != cudaDriverEntryPointSuccess || !fn) return cudaErrorNotSupported;
     encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
   }
-  const cuuint64_t strides[3] = {dims[0] * 4, dims[0] * 4 * dims[1], dims[0] * 4 * dims[1] * dims[2]};
+  const cuuint64_t slab = dims[0] * 4 * (pitch1 > 0 ? (cuuint64_t)pitch1 : dims[1]);
+  const cuuint64_t strides[3] = {dims[0] * 4, slab, slab * dims[2]};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult cr = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<void *>(base), dims, strides, box, estr,
                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,

@@ -8,8 +8,9 @@
 //
 // Work decomposition: the NI x NI input matrix of a frequency is split into
 // ST x ST super-tiles; only super-tiles on or above the diagonal are
-// computed.  A CTA owns one super-tile for CT channels and a slice of the
-// blocks; each thread owns a T x T register tile of accumulators for one
+// computed, and on the diagonal only the register tiles that reach the upper
+// triangle.  A CTA owns one super-tile for CT channels and a slice of the
+// blocks; each thread owns an 8 x TB register tile of accumulators for one
 // channel.  Spectra rows of the super-tile are staged in shared memory.
 //
 // Accumulators: acc[ks][freq][stpair][ST][ST][N] (float2), summed over the
@@ -25,57 +26,94 @@
 
 namespace gx {
 
-template <int T, int ST, int CT>
-__host__ __device__ constexpr int xmac_consumers() { return CT * (ST / T) * (ST / T); }
-
-// One CTA: super-tile pair blockIdx.x (upper triangle, row-major) of frequency
-// f for CT channels from c0 = blockIdx.y CT, over the blocks of K-split slice
-// ks.  One producer warp (the last) loads each stage -- KB blocks x ST rows x
-// CT channels of the I and (off the diagonal) J rows -- with one TMA tile per
-// operand into an NSTAGE ring; the consumer warps multiply from shared memory
-// and free each stage with one arrival per warp, so no CTA-wide barrier
-// separates the stages.  Every wait is bounded (kWaitLimitNs): on expiry the
-// CTA records a status in *err (when given), drains the copies it issued and
-// adds nothing.
-template <int T, int ST, int CT, int KB, int NSTAGE, int UNR = 1>
-__global__ void __launch_bounds__(xmac_consumers<T, ST, CT>() + 32, 1)
-xmac_fp32_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int N, int nsuper, int ks_count,
-                 int kper, float2 *__restrict__ acc, int *__restrict__ err)
+// Register tiles of a super-tile pair: kTA rows by TB columns.  On the diagonal
+// only those that reach the upper triangle (in whole groups of kTA rows).
+constexpr int kTA = 8;
+template <int TB, int ST, bool DIAG>
+__host__ __device__ constexpr int xmac_tiles()
 {
-  constexpr int NT = ST / T;            // register tiles per super-tile side
-  constexpr int NC = xmac_consumers<T, ST, CT>();
-  constexpr int NCW = NC / 32;          // consumer warps
+  int n = 0;
+  for (int i = 0; i < ST / kTA; i++) n += DIAG ? (ST - kTA * i) / TB : ST / TB;
+  return n;
+}
+// Consumer warps of a CTA: two tiles by 16 channels each.
+template <int TB, int ST, int CT, bool DIAG>
+__host__ __device__ constexpr int xmac_warps() { return xmac_tiles<TB, ST, DIAG>() / 2 * (CT / 16); }
+
+// One CTA: super-tile pair blockIdx.x (DIAG: the pairs on the diagonal, else
+// those above it, row-major) of frequency f for CT channels from c0 =
+// blockIdx.y CT, over the blocks of K-split slice ks.  Stages -- KB blocks x ST
+// rows x CT channels of the I and (off the diagonal) J rows, one TMA tile per
+// operand -- go round an NSTAGE ring: the warp that is last to finish with a
+// stage loads the next one into its place, so there is neither a producer warp
+// (a 21st warp would cost every thread of a 20-warp CTA 16 registers) nor a
+// barrier between the stages.  accumulate 0: the sums are stored, not added to
+// what acc holds.  Every wait is bounded (kWaitLimitNs): on expiry the CTA
+// records a status in *err (when given), drains the copies it issued and adds
+// nothing.
+//
+// What bounds it: the FMA pipe.  Only the register tiles that reach the upper
+// triangle have threads (32 inputs: 20 tiles of 8 x 4; a thread for each 8 x 8
+// tile of the square left 6 of 16 idle), and 8 x 4 tiles let 20 warps an SM hide
+// the shared-memory latency.  64 stations, 4096 channels, 125 blocks: 5.41 ->
+// 2.77 ms, 26 of the 36 T FMA lanes a second that 128 a clock are (16 stations,
+// 6250 blocks: 2.81 -> 1.18 ms, 28 of them).
+template <int TB, int ST, int CT, int KB, int NSTAGE, bool DIAG, int MINB>
+__global__ void __launch_bounds__(xmac_warps<TB, ST, CT, DIAG>() * 32, MINB)
+xmac_fp32_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int N, int nsuper, int ks_count,
+                 int kper, float2 *__restrict__ acc, int accumulate, int *__restrict__ err)
+{
+  constexpr int NCW = xmac_warps<TB, ST, CT, DIAG>();
+  constexpr int NTILE = xmac_tiles<TB, ST, DIAG>();
   constexpr int STAGE = KB * ST * CT;   // float2 per stage per operand
+  static_assert(NTILE % 2 == 0 && CT % 16 == 0 && ST % kTA == 0 && kTA % TB == 0, "a warp takes two tiles by 16 channels");
   extern __shared__ __align__(128) float2 xsm[];
   float2 *sI = xsm;                     // [NSTAGE][KB][ST][CT]
-  float2 *sJ = xsm + NSTAGE * STAGE;    // [NSTAGE][KB][ST][CT]
-  uint64_t *full = reinterpret_cast<uint64_t *>(sJ + NSTAGE * STAGE);
-  uint64_t *empty = full + NSTAGE;
-  volatile int *s_abort = reinterpret_cast<volatile int *>(empty + NSTAGE);
+  float2 *sJ = DIAG ? sI : xsm + NSTAGE * STAGE;
+  uint64_t *full = reinterpret_cast<uint64_t *>(xsm + (DIAG ? 1 : 2) * NSTAGE * STAGE);
+  int *s_done = reinterpret_cast<int *>(full + NSTAGE);   // warps done with each stage's current contents
+  volatile int *s_issued = s_done + NSTAGE;
+  volatile int *s_abort = s_done + NSTAGE + 1;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int stp = blockIdx.x;           // super-tile pair index
   const int c0 = blockIdx.y * CT;
   const int f = blockIdx.z / ks_count;
   const int ks = blockIdx.z % ks_count;
-  int SI = 0, rem = stp;
-  while (rem >= nsuper - SI) { rem -= nsuper - SI; SI++; }
-  const int SJ = SI + rem;
+  int SI, SJ;
+  if (DIAG) {
+    SI = SJ = blockIdx.x;
+  } else {
+    int rem = blockIdx.x;
+    SI = 0;
+    while (rem >= nsuper - 1 - SI) { rem -= nsuper - 1 - SI; SI++; }
+    SJ = SI + 1 + rem;
+  }
+  const int stp = SI * nsuper - SI * (SI - 1) / 2 + (SJ - SI);   // place among all upper pairs
   const int I0 = SI * ST, J0 = SJ * ST;
-  const bool diag = (SI == SJ);
 
   // slices start on stage boundaries (kper is a multiple of KB); the last
   // stage may reach past nblk, where the copies read zeros
   const int kb0 = ks * kper, kb1 = min(nblk, kb0 + kper);
   const int nstages = (kb1 > kb0) ? (kb1 - kb0 + KB - 1) / KB : 0;
 
+  auto load_stage = [&](int st) {   // one thread
+    const int b = st % NSTAGE, k = kb0 + st * KB;
+    const uint32_t bar = smem_u32(full + b);
+    mbar_expect_tx(bar, (DIAG ? 1u : 2u) * (uint32_t)(STAGE * sizeof(float2)));
+    tma_load_4d(smem_u32(sI + b * STAGE), &spec_map, 2 * c0, I0, k, f, bar);
+    if (!DIAG) tma_load_4d(smem_u32(sJ + b * STAGE), &spec_map, 2 * c0, J0, k, f, bar);
+    *s_issued = st + 1;   // stages are issued in order
+  };
   if (tid == 0) {
     for (int i = 0; i < NSTAGE; i++) {
       mbar_init(smem_u32(full + i), 1);
-      mbar_init(smem_u32(empty + i), NCW);
+      s_done[i] = 0;
     }
     *s_abort = 0;
+    *s_issued = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    fence_proxy_async_smem();
+    for (int i = 0; i < NSTAGE && i < nstages; i++) load_stage(i);
   }
   __syncthreads();
   auto abort_with = [&](int code) {
@@ -83,47 +121,23 @@ xmac_fp32_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int N, 
     if (err) atomicExch(err, code);
   };
 
-  if (warp == NCW) {
-    // ---- producer
-    if (lane == 0) {
-      const uint32_t bytes = (diag ? 1u : 2u) * (uint32_t)(STAGE * sizeof(float2));
-      int issued = 0;
-      for (int st = 0; st < nstages; st++) {
-        if (*s_abort) break;
-        const int b = st % NSTAGE;
-        if (st >= NSTAGE && !mbar_wait(smem_u32(empty + b), (uint32_t)(st / NSTAGE - 1) & 1u)) {
-          abort_with(13);
-          break;
-        }
-        const uint32_t bar = smem_u32(full + b);
-        mbar_expect_tx(bar, bytes);
-        const int k = kb0 + st * KB;
-        tma_load_4d(smem_u32(sI + b * STAGE), &spec_map, 2 * c0, I0, k, f, bar);
-        if (!diag) tma_load_4d(smem_u32(sJ + b * STAGE), &spec_map, 2 * c0, J0, k, f, bar);
-        issued = st + 1;
-      }
-      if (*s_abort) {
-        // drain: the copies this CTA issued land before it exits (bounded)
-        for (int b = 0; b < NSTAGE && b < issued; b++) {
-          const int ulast = b + ((issued - 1 - b) / NSTAGE) * NSTAGE;
-          mbar_wait(smem_u32(full + b), (uint32_t)(ulast / NSTAGE) & 1u);
-        }
-      }
-    }
-    return;
+  // ---- consumers: a kTA x TB register tile of one channel; a warp takes two
+  // neighbouring tiles (mostly of the same rows) by 16 channels, so that its
+  // row loads are whole 128-byte lines
+  const int c = (warp / (NTILE / 2)) * 16 + (lane & 15);
+  int ti = 0, tj = 2 * (warp % (NTILE / 2)) + (lane >> 4);
+  if (DIAG) {
+    while (tj >= (ST - kTA * ti) / TB) { tj -= (ST - kTA * ti) / TB; ti++; }
+    tj += kTA / TB * ti;
+  } else {
+    ti = tj / (ST / TB);
+    tj %= ST / TB;
   }
-
-  // ---- consumers: a T x T register tile of one channel
-  const int c = tid % CT;
-  const int p = tid / CT;
-  const int ti = p / NT, tj = p % NT;
-  const float2 *sJread = diag ? sI : sJ;
-  float2 acc2[T][T];   // (Re, Im) of each product sum, one register pair for the f32x2 FMAs
+  float2 acc2[kTA][TB];   // (Re, Im) of each product sum, one register pair for the f32x2 FMAs
 #pragma unroll
-  for (int a = 0; a < T; a++)
+  for (int a = 0; a < kTA; a++)
 #pragma unroll
-    for (int b = 0; b < T; b++) acc2[a][b] = make_float2(0.f, 0.f);
-  const bool compute = !diag || (ti <= tj);   // lower tiles of diagonal super-tiles are redundant
+    for (int b = 0; b < TB; b++) acc2[a][b] = make_float2(0.f, 0.f);
   bool ok = true;
   for (int st = 0; st < nstages; st++) {
     const int buf = st % NSTAGE;
@@ -132,53 +146,73 @@ xmac_fp32_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int N, 
       ok = false;
       break;
     }
-    if (compute) {
-      const float2 *bi_ = sI + buf * STAGE;
-      const float2 *bj_ = sJread + buf * STAGE;
-#pragma unroll UNR
-      for (int kk = 0; kk < KB; kk++) {
-        float2 xi[T], xj[T];
+    const float2 *bi_ = sI + buf * STAGE + ti * kTA * CT + c;
+    const float2 *bj_ = sJ + buf * STAGE + tj * TB * CT + c;
+#pragma unroll 1
+    for (int kk = 0; kk < KB; kk++) {
+      // xi * conj(xj) as two paired FMAs (one f32x2 instruction each on
+      // sm_100): Re += xi.x xj.x then xi.y xj.y; Im += xi.y xj.x then -xi.x xj.y,
+      // the same operations in the same order as four scalar FMAs.
+      float2 bx[TB], by[TB];
 #pragma unroll
-        for (int r = 0; r < T; r++) {
-          xi[r] = bi_[(kk * ST + ti * T + r) * CT + c];
-          xj[r] = bj_[(kk * ST + tj * T + r) * CT + c];
-        }
-        // xi * conj(xj) as two paired FMAs (one f32x2 instruction each on
-        // sm_100): Re += xi.x xj.x then xi.y xj.y; Im += xi.y xj.x then -xi.x xj.y,
-        // the same operations in the same order as four scalar FMAs.
-        float2 xs[T], bx[T], by[T];
+      for (int r = 0; r < TB; r++) {
+        const float2 xj = bj_[(kk * ST + r) * CT];
+        bx[r] = make_float2(xj.x, xj.x);
+        by[r] = make_float2(xj.y, xj.y);
+      }
 #pragma unroll
-        for (int r = 0; r < T; r++) {
-          xs[r] = make_float2(xi[r].y, -xi[r].x);
-          bx[r] = make_float2(xj[r].x, xj[r].x);
-          by[r] = make_float2(xj[r].y, xj[r].y);
-        }
+      for (int a = 0; a < kTA; a++) {
+        const float2 xi = bi_[(kk * ST + a) * CT];
+        const float2 xs = make_float2(xi.y, -xi.x);
 #pragma unroll
-        for (int a = 0; a < T; a++)
+        for (int b = 0; b < TB; b++) acc2[a][b] = __ffma2_rn(xi, bx[b], acc2[a][b]);
 #pragma unroll
-          for (int b = 0; b < T; b++) {
-            acc2[a][b] = __ffma2_rn(xi[a], bx[b], acc2[a][b]);
-            acc2[a][b] = __ffma2_rn(xs[a], by[b], acc2[a][b]);
-          }
+        for (int b = 0; b < TB; b++) acc2[a][b] = __ffma2_rn(xs, by[b], acc2[a][b]);
       }
     }
     __syncwarp();
-    if (lane == 0) mbar_arrive(smem_u32(empty + buf));   // the stage may be reloaded
-  }
-  if (!ok || !compute || c0 + c >= N) return;
-  const int nfreqs = gridDim.z / ks_count;
-  const size_t base = (((size_t)ks * nfreqs + f) * gridDim.x + stp) * (size_t)ST * ST;
-#pragma unroll
-  for (int a = 0; a < T; a++)
-#pragma unroll
-    for (int b = 0; b < T; b++) {
-      const int ii = ti * T + a, jj = tj * T + b;
-      float2 *dst = acc + (base + (size_t)ii * ST + jj) * N + c0 + c;
-      float2 v = *dst;
-      v.x += acc2[a][b].x;
-      v.y += acc2[a][b].y;
-      *dst = v;
+    if (lane == 0) {
+      // done with the stage: the last warp to be (its acquire follows every
+      // other's release, so all reads of the stage precede the copy) refills it
+      int before;
+      asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;" : "=r"(before) : "r"(smem_u32(s_done + buf)) : "memory");
+      if (before == NCW - 1 && st + NSTAGE < nstages && !*s_abort) {
+        s_done[buf] = 0;
+        load_stage(st + NSTAGE);
+      }
     }
+  }
+  if (*s_abort) ok = false;
+  if (__syncthreads_or(!ok)) {
+    // drain: the copies this CTA issued land before it exits (bounded)
+    if (tid == 0) {
+      const int issued = *s_issued;
+      for (int b = 0; b < NSTAGE && b < issued; b++) {
+        const int ulast = b + ((issued - 1 - b) / NSTAGE) * NSTAGE;
+        mbar_wait(smem_u32(full + b), (uint32_t)(ulast / NSTAGE) & 1u);
+      }
+    }
+    __syncthreads();
+    return;
+  }
+  if (c0 + c >= N) return;
+  const int nfreqs = gridDim.z / ks_count, npairs = nsuper * (nsuper + 1) / 2;
+  const size_t base = (((size_t)ks * nfreqs + f) * npairs + stp) * (size_t)ST * ST;
+  float2 *tile = acc + (base + (size_t)(ti * kTA) * ST + tj * TB) * N + c0 + c;
+#pragma unroll
+  for (int a = 0; a < kTA; a++) {
+    float2 old[TB];   // a row's loads together: one by one, behind the stores, their latency was a tenth of a pass
+    if (accumulate) {
+#pragma unroll
+      for (int b = 0; b < TB; b++) old[b] = tile[(size_t)(a * ST + b) * N];
+    }
+#pragma unroll
+    for (int b = 0; b < TB; b++) {
+      float2 v = acc2[a][b];
+      if (accumulate) v = make_float2(v.x + old[b].x, v.y + old[b].y);
+      tile[(size_t)(a * ST + b) * N] = v;
+    }
+  }
 }
 
 // Sum of weights over the blocks of one chunk (Core::processdata baseline
@@ -186,30 +220,28 @@ xmac_fp32_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int N, 
 // Weight sums over a pass of blocks: item i < nstations sums station row i;
 // item nstations + k sums the products of rows pairs[k] (or row pairs[k].x
 // alone when pairs[k].y < 0).
-__global__ void weights_kernel(const float *__restrict__ w, int nblk, int nstations,
-                               const int2 *__restrict__ pairs, int npairs, float *__restrict__ wacc)
+constexpr int kWeightThreads = 1024;
+__global__ void __launch_bounds__(kWeightThreads)
+weights_kernel(const float *__restrict__ w, int nblk, int nstations, const int2 *__restrict__ pairs, int npairs,
+               float *__restrict__ wacc)
 {
-  __shared__ float red[256];
+  __shared__ float red[kWeightThreads / 32];
   const int item = blockIdx.x;  // [0, nstations): station sums; then baseline products
+  const int2 pr = item < nstations ? make_int2(item, -1) : pairs[item - nstations];
+  const float *x = w + (size_t)pr.x * nblk;
+  const float *y = pr.y < 0 ? nullptr : w + (size_t)pr.y * nblk;   // null: one row alone
   float sum = 0.f;
-  if (item < nstations) {
-    for (int b = threadIdx.x; b < nblk; b += blockDim.x) sum += w[(size_t)item * nblk + b];
-  } else {
-    const int2 pr = pairs[item - nstations];
-    if (pr.y < 0) {   // one row alone (a per-band weight row)
-      for (int b = threadIdx.x; b < nblk; b += blockDim.x) sum += w[(size_t)pr.x * nblk + b];
-    } else {
-      for (int b = threadIdx.x; b < nblk; b += blockDim.x)
-        sum += w[(size_t)pr.x * nblk + b] * w[(size_t)pr.y * nblk + b];
-    }
-  }
-  red[threadIdx.x] = sum;
+  // several loads in flight: a CTA reads whole rows, and there are few CTAs
+#pragma unroll 4
+  for (int b = threadIdx.x; b < nblk; b += kWeightThreads) sum += y ? x[b] * y[b] : x[b];
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sum;
   __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-    __syncthreads();
+  if (threadIdx.x < 32) {
+    sum = red[threadIdx.x];
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (threadIdx.x == 0) wacc[item] += sum;
   }
-  if (threadIdx.x == 0) wacc[item] += red[0];
 }
 
 // Result array assembly (Core result layout).
@@ -241,67 +273,76 @@ __global__ void finalise_weights_kernel(const WeightEntry *__restrict__ we, int 
 
 // ------------------------------------------------------------------ launchers
 
-template <int T, int ST, int CT, int KB, int NSTAGE, int UNR = 1>
-static cudaError_t launch_t(const float2 *spec, int nblk, int NI, int N, int nfreqs, int ks, float2 *acc, int *err,
-                            cudaStream_t st)
+template <int TB, int ST, int CT, int KB, int NSTAGE, bool DIAG, int MINB>
+static cudaError_t launch_t(const float2 *spec, int nblk, int rows, int NI, int N, int nfreqs, int ks, float2 *acc,
+                            int accumulate, int *err, cudaStream_t st)
 {
   const int nsuper = (NI + ST - 1) / ST;
-  const int npairs = nsuper * (nsuper + 1) / 2;
-  const size_t sm = sizeof(float2) * 2 * NSTAGE * KB * ST * CT + 2 * NSTAGE * sizeof(uint64_t) + 16;
+  const int npairs = DIAG ? nsuper : nsuper * (nsuper - 1) / 2;
+  if (npairs == 0) return cudaSuccess;
+  const size_t sm = sizeof(float2) * (DIAG ? 1 : 2) * NSTAGE * KB * ST * CT + NSTAGE * (sizeof(uint64_t) + sizeof(int)) + 16;
   // spec[freq][block][row][channel] float2 as a 4-D FP32 tensor: {2N floats,
-  // NI rows, nblk blocks, nfreqs}; one box = KB blocks x ST rows x CT channels
+  // rows in use (the others of the NI are not read), nblk blocks, nfreqs}; one
+  // box = KB blocks x ST rows x CT channels
   CUtensorMap map;
-  const cuuint64_t dims[4] = {(cuuint64_t)(2 * N), (cuuint64_t)NI, (cuuint64_t)nblk, (cuuint64_t)nfreqs};
+  const cuuint64_t dims[4] = {(cuuint64_t)(2 * N), (cuuint64_t)rows, (cuuint64_t)nblk, (cuuint64_t)nfreqs};
   const cuuint32_t box[4] = {(cuuint32_t)(2 * CT), (cuuint32_t)ST, (cuuint32_t)KB, 1};
-  cudaError_t e = tma_map_f32_4d(&map, spec, dims, box);
+  cudaError_t e = tma_map_f32_4d(&map, spec, dims, box, NI);
   if (e != cudaSuccess) return e;
-  e = smem_opt_in((const void *)xmac_fp32_kernel<T, ST, CT, KB, NSTAGE, UNR>, sm);
+  auto kernel = xmac_fp32_kernel<TB, ST, CT, KB, NSTAGE, DIAG, MINB>;
+  e = smem_opt_in((const void *)kernel, sm);
   if (e != cudaSuccess) return e;
-  // slices of whole stages, on 16-block boundaries for every variant (KB 8
-  // or 16), so that the variants add the same blocks into each slice
+  // slices of whole stages, on 16-block boundaries for every variant, so that
+  // the variants add the same blocks into each slice
   static_assert(16 % KB == 0, "slice boundaries must be whole stages");
   const int kper = ((nblk + ks - 1) / ks + 15) / 16 * 16;
   // super-tile pairs fastest: the pairs that share a channel group's spectra run together
   dim3 grid(npairs, (N + CT - 1) / CT, nfreqs * ks);
-  xmac_fp32_kernel<T, ST, CT, KB, NSTAGE, UNR>
-      <<<grid, xmac_consumers<T, ST, CT>() + 32, sm, st>>>(map, nblk, N, nsuper, ks, kper, acc, err);
+  kernel<<<grid, xmac_warps<TB, ST, CT, DIAG>() * 32, sm, st>>>(map, nblk, N, nsuper, ks, kper, acc, accumulate, err);
   return cudaGetLastError();
 }
 
+// Channels per CTA: 20 warps of 20 tiles by 32 channels where one super-tile
+// holds every input (16 stations, 2-bit, 6250 blocks: X stage 2.81 -> 1.18 ms;
+// 16 channels and two CTAs an SM 1.34, 8 x 8 tiles 1.66 before longer passes),
+// as on the diagonal of larger ones; 12 warps of 6 tiles by 64 channels for 16
+// rows (11 stations: 0.42 ms, two CTAs of 32 channels 0.54, the square of 4 x 4
+// tiles 0.66); two warps of two tiles by 32 channels for 8 rows (4 stations, 25000
+// blocks: 0.17 ms, 64 channels 0.18, 4 x 4 tiles 0.36).
 XmacShape xmac_shape(int NI)
 {
   XmacShape s;
-  if (NI <= 8) { s.T = 4; s.ST = 8; s.CT = 32; }
-  else if (NI <= 16) { s.T = 4; s.ST = 16; s.CT = 16; }
-  else { s.T = 8; s.ST = 32; s.CT = 16; }
+  s.T = kTA;
+  if (NI <= 8) { s.ST = 8; s.CT = 32; }
+  else if (NI <= 16) { s.ST = 16; s.CT = 64; }
+  else { s.ST = 32; s.CT = NI <= 32 ? 32 : 16; }
   s.nsuper = (NI + s.ST - 1) / s.ST;
   s.npairs = s.nsuper * (s.nsuper + 1) / 2;
   return s;
 }
 
-cudaError_t xmac_fp32_launch(const float2 *spec, int nblk, int NI, int N, int nfreqs, int ks, float2 *acc, int *err,
-                             cudaStream_t st, int variant)
+cudaError_t xmac_fp32_launch(const float2 *spec, int nblk, int rows, int NI, int N, int nfreqs, int ks, float2 *acc,
+                             int accumulate, int *err, cudaStream_t st, int variant)
 {
-  // every variant keeps the register tile T and super-tile ST of the shape
-  // (the accumulator layout) and 192 KB of stages; variant 1 trades channels
-  // per CTA against blocks per stage (or doubles the channels)
-  XmacShape s = xmac_shape(NI);
-  if (s.ST == 8)
-    return variant == 1 ? launch_t<4, 8, 64, 8, 3>(spec, nblk, NI, N, nfreqs, ks, acc, err, st)
-                        : launch_t<4, 8, 32, 8, 3>(spec, nblk, NI, N, nfreqs, ks, acc, err, st);
-  if (s.ST == 16)
-    return variant == 1 ? launch_t<4, 16, 32, 8, 3>(spec, nblk, NI, N, nfreqs, ks, acc, err, st)
-                        : launch_t<4, 16, 16, 8, 3>(spec, nblk, NI, N, nfreqs, ks, acc, err, st);
-  // 8 x 8 register tiles of 32-row super-tiles, 16 channels per CTA; the
-  // block loop is not unrolled (unrolled by 2 or 4 it measured 3-9% slower)
-  return variant == 1 ? launch_t<8, 32, 8, 16, 3>(spec, nblk, NI, N, nfreqs, ks, acc, err, st)
-                      : launch_t<8, 32, 16, 8, 3>(spec, nblk, NI, N, nfreqs, ks, acc, err, st);
+  // every variant keeps the super-tile ST of the shape (the accumulator
+  // layout); variant 1 takes half (or twice) the channels per CTA
+  const XmacShape s = xmac_shape(NI);
+#define GX_XMAC(TB, ST, CT, KB, DG, MB) \
+  launch_t<TB, ST, CT, KB, 3, DG, MB>(spec, nblk, rows, NI, N, nfreqs, ks, acc, accumulate, err, st)
+  if (s.ST == 8) return variant == 1 ? GX_XMAC(4, 8, 64, 4, true, 4) : GX_XMAC(4, 8, 32, 8, true, 4);
+  if (s.ST == 16) return variant == 1 ? GX_XMAC(4, 16, 32, 8, true, 2) : GX_XMAC(4, 16, 64, 8, true, 1);
+  cudaError_t e = variant == 1 ? GX_XMAC(4, 32, 16, 8, true, 2) : GX_XMAC(4, 32, 32, 8, true, 1);
+  if (e != cudaSuccess) return e;
+  // above the diagonal: 8 x 8 tiles, half the shared-memory reads a product of
+  // 8 x 4 (64 stations, 125 blocks: 1.98 against 2.06 ms)
+  return variant == 1 ? GX_XMAC(4, 32, 16, 8, false, 1) : GX_XMAC(8, 32, 16, 8, false, 1);
+#undef GX_XMAC
 }
 
 cudaError_t weights_launch(const float *w, int nblk, int nstations, const int2 *pairs, int npairs, float *wacc,
                            cudaStream_t st)
 {
-  weights_kernel<<<nstations + npairs, 256, 0, st>>>(w, nblk, nstations, pairs, npairs, wacc);
+  weights_kernel<<<nstations + npairs, kWeightThreads, 0, st>>>(w, nblk, nstations, pairs, npairs, wacc);
   return cudaGetLastError();
 }
 

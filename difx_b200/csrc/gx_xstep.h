@@ -38,7 +38,10 @@ struct XmacShape {
 XmacShape xmac_shape(int NI);
 
 // 4-D FP32 tensor map over a dense array (dims innermost first), box `box`.
-cudaError_t tma_map_f32_4d(CUtensorMap *map, const void *base, const cuuint64_t dims[4], const cuuint32_t box[4]);
+// pitch1: rows (dimension 1) from one index of dimension 2 to the next, where
+// they are more than dims[1] (0: dims[1]).
+cudaError_t tma_map_f32_4d(CUtensorMap *map, const void *base, const cuuint64_t dims[4], const cuuint32_t box[4],
+                           int pitch1 = 0);
 
 size_t fstep_smem_bytes(const DevJob &J, int nrf, int nslots);
 // The paired-band F-step (gx_fstep_pair.cuh): whether it takes this job, blocks
@@ -53,13 +56,15 @@ cudaError_t fstep_pair_launch(const DevJob &J, const DevStation *stations, const
 cudaError_t fstep_launch(const DevJob &J, const DevStation *stations, int maxnrf, const SubintArrays &S,
                          int blk0, int nblk, int nslots, float2 *spec, float *weights, BlockParam *bp,
                          cudaStream_t st, const PcalFuse *pf = nullptr, bool *pcal_done = nullptr);
-// FP32 X-step over one pass of blocks; *err (may be null) receives a nonzero
-// status if a wait of the kernel expired.  variant: the launch shape (0: the
-// default channel tile and stage depth; 1: the other one of the shape class,
-// kXmacVariants in all); the sums are the same for every variant.
+// FP32 X-step over one pass of blocks, NI spectra rows of which the first
+// `rows` are in use; accumulate 0: acc is overwritten (its upper tiles), not
+// added to.  *err (may be null) receives a nonzero status if a wait of the
+// kernel expired.  variant: the launch shape (0: the default channels per CTA;
+// 1: the other one of the shape class, kXmacVariants in all); the sums are the
+// same for every variant.
 constexpr int kXmacVariants = 2;
-cudaError_t xmac_fp32_launch(const float2 *spec, int nblk, int NI, int N, int nfreqs, int ks, float2 *acc, int *err,
-                             cudaStream_t st, int variant = 0);
+cudaError_t xmac_fp32_launch(const float2 *spec, int nblk, int rows, int NI, int N, int nfreqs, int ks, float2 *acc,
+                             int accumulate, int *err, cudaStream_t st, int variant = 0);
 cudaError_t weights_launch(const float *w, int nblk, int nstations, const int2 *pairs, int npairs, float *wacc,
                            cudaStream_t st);
 // Entries [start, end) of the tensor-core product table (sorted by freq, then a)
