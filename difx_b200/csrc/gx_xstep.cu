@@ -50,7 +50,7 @@ __host__ __device__ constexpr int xmac_warps() { return xmac_tiles<TB, ST, DIAG>
 // barrier between the stages.  accumulate 0: the sums are stored, not added to
 // what acc holds.  Every wait is bounded (kWaitLimitNs): on expiry the CTA
 // records a status in *err (when given), drains the copies it issued and adds
-// nothing.
+// nothing more.
 //
 // What bounds it: the FMA pipe.  Only the register tiles that reach the upper
 // triangle have threads (32 inputs: 20 tiles of 8 x 4; a thread for each 8 x 8
@@ -58,7 +58,10 @@ __host__ __device__ constexpr int xmac_warps() { return xmac_tiles<TB, ST, DIAG>
 // the shared-memory latency.  64 stations, 4096 channels, 125 blocks: 5.41 ->
 // 2.77 ms, 26 of the 36 T FMA lanes a second that 128 a clock are (16 stations,
 // 6250 blocks: 2.81 -> 1.18 ms, 28 of them).
-template <int TB, int ST, int CT, int KB, int NSTAGE, bool DIAG, int MINB>
+// The sums of a product stay short: after kRun blocks in one register, TWO
+// register levels (where the shape leaves the registers) or the accumulators in
+// memory take them over, so the FP32 error does not grow with the pass.
+template <int TB, int ST, int CT, int KB, int NSTAGE, bool DIAG, int MINB, bool TWO>
 __global__ void __launch_bounds__(xmac_warps<TB, ST, CT, DIAG>() * 32, MINB)
 xmac_fp32_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int N, int nsuper, int ks_count,
                  int kper, float2 *__restrict__ acc, int accumulate, int *__restrict__ err)
@@ -66,6 +69,8 @@ xmac_fp32_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int N, 
   constexpr int NCW = xmac_warps<TB, ST, CT, DIAG>();
   constexpr int NTILE = xmac_tiles<TB, ST, DIAG>();
   constexpr int STAGE = KB * ST * CT;   // float2 per stage per operand
+  constexpr int kRun = TWO ? 128 : 256;
+  static_assert(kRun % KB == 0, "runs of whole stages");
   static_assert(NTILE % 2 == 0 && CT % 16 == 0 && ST % kTA == 0 && kTA % TB == 0, "a warp takes two tiles by 16 channels");
   extern __shared__ __align__(128) float2 xsm[];
   float2 *sI = xsm;                     // [NSTAGE][KB][ST][CT]
@@ -138,50 +143,102 @@ xmac_fp32_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int N, 
   for (int a = 0; a < kTA; a++)
 #pragma unroll
     for (int b = 0; b < TB; b++) acc2[a][b] = make_float2(0.f, 0.f);
-  bool ok = true;
-  for (int st = 0; st < nstages; st++) {
-    const int buf = st % NSTAGE;
-    if (!mbar_wait(smem_u32(full + buf), (uint32_t)(st / NSTAGE) & 1u) || *s_abort) {
-      abort_with(14);
-      ok = false;
-      break;
-    }
-    const float2 *bi_ = sI + buf * STAGE + ti * kTA * CT + c;
-    const float2 *bj_ = sJ + buf * STAGE + tj * TB * CT + c;
-#pragma unroll 1
-    for (int kk = 0; kk < KB; kk++) {
-      // xi * conj(xj) as two paired FMAs (one f32x2 instruction each on
-      // sm_100): Re += xi.x xj.x then xi.y xj.y; Im += xi.y xj.x then -xi.x xj.y,
-      // the same operations in the same order as four scalar FMAs.
-      float2 bx[TB], by[TB];
+  float2 tot[TWO ? kTA : 1][TWO ? TB : 1];   // the finished runs' sums
+  if constexpr (TWO) {
 #pragma unroll
-      for (int r = 0; r < TB; r++) {
-        const float2 xj = bj_[(kk * ST + r) * CT];
-        bx[r] = make_float2(xj.x, xj.x);
-        by[r] = make_float2(xj.y, xj.y);
-      }
+    for (int a = 0; a < kTA; a++)
 #pragma unroll
-      for (int a = 0; a < kTA; a++) {
-        const float2 xi = bi_[(kk * ST + a) * CT];
-        const float2 xs = make_float2(xi.y, -xi.x);
-#pragma unroll
-        for (int b = 0; b < TB; b++) acc2[a][b] = __ffma2_rn(xi, bx[b], acc2[a][b]);
-#pragma unroll
-        for (int b = 0; b < TB; b++) acc2[a][b] = __ffma2_rn(xs, by[b], acc2[a][b]);
-      }
-    }
-    __syncwarp();
-    if (lane == 0) {
-      // done with the stage: the last warp to be (its acquire follows every
-      // other's release, so all reads of the stage precede the copy) refills it
-      int before;
-      asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;" : "=r"(before) : "r"(smem_u32(s_done + buf)) : "memory");
-      if (before == NCW - 1 && st + NSTAGE < nstages && !*s_abort) {
-        s_done[buf] = 0;
-        load_stage(st + NSTAGE);
-      }
-    }
+      for (int b = 0; b < TB; b++) tot[a][b] = make_float2(0.f, 0.f);
   }
+  const int nfreqs = gridDim.z / ks_count, npairs = nsuper * (nsuper + 1) / 2;
+  float2 *tile = acc + ((((size_t)ks * nfreqs + f) * npairs + stp) * (size_t)ST * ST + (ti * kTA) * ST + tj * TB) * N + c0 + c;
+  // adds (or stores) the tile's sums x
+  auto put = [&](const float2 (&x)[kTA][TB], bool add) {
+    if (c0 + c >= N) return;
+    float2 *t = tile;
+    asm volatile("" : "+l"(t));   // no addresses formed ahead: they would cost the loop its registers
+#pragma unroll
+    for (int a = 0; a < kTA; a++, t += (size_t)ST * N) {
+      float2 old[TB];   // a row's loads together: one by one, behind the stores, their latency was a tenth of a pass
+      if (add) {
+#pragma unroll
+        for (int b = 0; b < TB; b++) old[b] = t[(size_t)b * N];
+      }
+#pragma unroll
+      for (int b = 0; b < TB; b++) {
+        float2 v = x[a][b];
+        if (add) v = make_float2(v.x + old[b].x, v.y + old[b].y);
+        t[(size_t)b * N] = v;
+      }
+    }
+  };
+  bool ok = true, add = accumulate != 0;
+  int st = 0;
+#pragma unroll 1
+  do {
+    const int run = min(nstages, st + kRun / KB);
+#pragma unroll 1
+    for (; st < run; st++) {
+      const int buf = st % NSTAGE;
+      if (!mbar_wait(smem_u32(full + buf), (uint32_t)(st / NSTAGE) & 1u) || *s_abort) {
+        abort_with(14);
+        ok = false;
+        break;
+      }
+      const float2 *bi_ = sI + buf * STAGE + ti * kTA * CT + c;
+      const float2 *bj_ = sJ + buf * STAGE + tj * TB * CT + c;
+#pragma unroll 1
+      for (int kk = 0; kk < KB; kk++) {
+        // xi * conj(xj) as two paired FMAs (one f32x2 instruction each on
+        // sm_100): Re += xi.x xj.x then xi.y xj.y; Im += xi.y xj.x then -xi.x xj.y,
+        // the same operations in the same order as four scalar FMAs.
+        float2 bx[TB], by[TB];
+#pragma unroll
+        for (int r = 0; r < TB; r++) {
+          const float2 xj = bj_[(kk * ST + r) * CT];
+          bx[r] = make_float2(xj.x, xj.x);
+          by[r] = make_float2(xj.y, xj.y);
+        }
+#pragma unroll
+        for (int a = 0; a < kTA; a++) {
+          const float2 xi = bi_[(kk * ST + a) * CT];
+          const float2 xs = make_float2(xi.y, -xi.x);
+#pragma unroll
+          for (int b = 0; b < TB; b++) acc2[a][b] = __ffma2_rn(xi, bx[b], acc2[a][b]);
+#pragma unroll
+          for (int b = 0; b < TB; b++) acc2[a][b] = __ffma2_rn(xs, by[b], acc2[a][b]);
+        }
+      }
+      __syncwarp();
+      if (lane == 0) {
+        // done with the stage: the last warp to be (its acquire follows every
+        // other's release, so all reads of the stage precede the copy) refills it
+        int before;
+        asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;" : "=r"(before) : "r"(smem_u32(s_done + buf)) : "memory");
+        if (before == NCW - 1 && st + NSTAGE < nstages && !*s_abort) {
+          s_done[buf] = 0;
+          load_stage(st + NSTAGE);
+        }
+      }
+    }
+    if (!ok) break;
+    if constexpr (TWO) {
+#pragma unroll
+      for (int a = 0; a < kTA; a++)
+#pragma unroll
+        for (int b = 0; b < TB; b++) {
+          tot[a][b] = make_float2(tot[a][b].x + acc2[a][b].x, tot[a][b].y + acc2[a][b].y);
+          acc2[a][b] = make_float2(0.f, 0.f);
+        }
+    } else {
+      put(acc2, add);
+      add = true;
+#pragma unroll
+      for (int a = 0; a < kTA; a++)
+#pragma unroll
+        for (int b = 0; b < TB; b++) acc2[a][b] = make_float2(0.f, 0.f);
+    }
+  } while (st < nstages);
   if (*s_abort) ok = false;
   if (__syncthreads_or(!ok)) {
     // drain: the copies this CTA issued land before it exits (bounded)
@@ -195,24 +252,7 @@ xmac_fp32_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int N, 
     __syncthreads();
     return;
   }
-  if (c0 + c >= N) return;
-  const int nfreqs = gridDim.z / ks_count, npairs = nsuper * (nsuper + 1) / 2;
-  const size_t base = (((size_t)ks * nfreqs + f) * npairs + stp) * (size_t)ST * ST;
-  float2 *tile = acc + (base + (size_t)(ti * kTA) * ST + tj * TB) * N + c0 + c;
-#pragma unroll
-  for (int a = 0; a < kTA; a++) {
-    float2 old[TB];   // a row's loads together: one by one, behind the stores, their latency was a tenth of a pass
-    if (accumulate) {
-#pragma unroll
-      for (int b = 0; b < TB; b++) old[b] = tile[(size_t)(a * ST + b) * N];
-    }
-#pragma unroll
-    for (int b = 0; b < TB; b++) {
-      float2 v = acc2[a][b];
-      if (accumulate) v = make_float2(v.x + old[b].x, v.y + old[b].y);
-      tile[(size_t)(a * ST + b) * N] = v;
-    }
-  }
+  if constexpr (TWO) put(tot, add);
 }
 
 // Sum of weights over the blocks of one chunk (Core::processdata baseline
@@ -273,7 +313,7 @@ __global__ void finalise_weights_kernel(const WeightEntry *__restrict__ we, int 
 
 // ------------------------------------------------------------------ launchers
 
-template <int TB, int ST, int CT, int KB, int NSTAGE, bool DIAG, int MINB>
+template <int TB, int ST, int CT, int KB, int NSTAGE, bool DIAG, int MINB, bool TWO>
 static cudaError_t launch_t(const float2 *spec, int nblk, int rows, int NI, int N, int nfreqs, int ks, float2 *acc,
                             int accumulate, int *err, cudaStream_t st)
 {
@@ -289,7 +329,7 @@ static cudaError_t launch_t(const float2 *spec, int nblk, int rows, int NI, int 
   const cuuint32_t box[4] = {(cuuint32_t)(2 * CT), (cuuint32_t)ST, (cuuint32_t)KB, 1};
   cudaError_t e = tma_map_f32_4d(&map, spec, dims, box, NI);
   if (e != cudaSuccess) return e;
-  auto kernel = xmac_fp32_kernel<TB, ST, CT, KB, NSTAGE, DIAG, MINB>;
+  auto kernel = xmac_fp32_kernel<TB, ST, CT, KB, NSTAGE, DIAG, MINB, TWO>;
   e = smem_opt_in((const void *)kernel, sm);
   if (e != cudaSuccess) return e;
   // slices of whole stages, on 16-block boundaries for every variant, so that
@@ -328,8 +368,8 @@ cudaError_t xmac_fp32_launch(const float2 *spec, int nblk, int rows, int NI, int
   // layout); variant 1 takes half (or twice) the channels per CTA
   const XmacShape s = xmac_shape(NI);
 #define GX_XMAC(TB, ST, CT, KB, DG, MB) \
-  launch_t<TB, ST, CT, KB, 3, DG, MB>(spec, nblk, rows, NI, N, nfreqs, ks, acc, accumulate, err, st)
-  if (s.ST == 8) return variant == 1 ? GX_XMAC(4, 8, 64, 4, true, 4) : GX_XMAC(4, 8, 32, 8, true, 4);
+  launch_t<TB, ST, CT, KB, 3, DG, MB, (ST < 32)>(spec, nblk, rows, NI, N, nfreqs, ks, acc, accumulate, err, st)
+  if (s.ST == 8) return variant == 1 ? GX_XMAC(4, 8, 64, 4, true, 3) : GX_XMAC(4, 8, 32, 8, true, 4);
   if (s.ST == 16) return variant == 1 ? GX_XMAC(4, 16, 32, 8, true, 2) : GX_XMAC(4, 16, 64, 8, true, 1);
   cudaError_t e = variant == 1 ? GX_XMAC(4, 32, 16, 8, true, 2) : GX_XMAC(4, 32, 32, 8, true, 1);
   if (e != cudaSuccess) return e;
