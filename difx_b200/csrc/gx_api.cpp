@@ -868,6 +868,36 @@ static gx_status setup(gx_handle *h)
     }
   }
 
+  // Do the visibility rows cover every record?  (They are distinct.)  Then,
+  // with an entry for every float of the weight sections, nothing of the result
+  // has to be cleared before the finalise kernels (the phase-cal section that
+  // follows is written whole).
+  h->covered = false;
+  if (h->nbins == 0 && h->maxpc == 1 && d.nstations > 0) {
+    long long w0 = h->acofs_full[0];
+    for (int x : h->bwofs_full)
+      if (x >= 0) w0 = std::min<long long>(w0, x);
+    const long long covered = (long long)h->prods.size() * J.nchan + (long long)h->zprods.size() * h->nzchan;
+    if (covered == w0 + (h->acwofs_full[0] - h->acofs_full[0])) {
+      h->covered = true;
+      long long end = h->rl_full;
+      for (const PcalBand &P : h->pcal) end -= P.ntones;
+      const long long a0 = 2 * w0, a1 = 2LL * h->acofs_full[0], b0 = 2LL * h->acwofs_full[0], b1 = 2 * end;
+      std::vector<char> seen((size_t)(a1 - a0 + b1 - b0), 0);
+      auto at = [&](long long x) { return (size_t)(x < a1 ? x - a0 : a1 - a0 + x - b0); };
+      for (const WeightEntry &w : h->wents) seen[at(w.float_index)] = 1;
+      for (long long x = a0; x < b1; x = x + 1 == a1 ? b0 : x + 1)
+        if ((x < a1 || x >= b0) && !seen[at(x)]) {
+          WeightEntry w{};
+          w.float_index = x;
+          w.source = -1;
+          h->wents.push_back(w);
+        }
+    }
+  }
+  h->tc_upper = true;
+  for (const TcProdEntry &t : h->tcprods) h->tc_upper = h->tc_upper && t.b / 8 >= t.a / 8;
+
   if (h->nbins > 0) h->autoprods.assign(h->prods.begin() + ncross_prods, h->prods.end());
 
   // tensor-core finalising pass: entries grouped by (freq, a) row
@@ -1043,6 +1073,8 @@ static gx_status setup(gx_handle *h)
     // that the FP16 values and their split remainders stay in the normal range.
     double ms = 0;
     const int ncode = 1 << J.nbits;
+    J.lut_zero = 0;
+    for (int l = 0; l < ncode; l++) J.lut_zero |= lut[l] == 0.0f;
     for (int l = 0; l < ncode; l++) ms += (double)lut[l] * lut[l];
     ms /= ncode;
     const double rms_spec = std::sqrt(ms * J.fftlen * (J.cplx ? 2.0 : 1.0));
@@ -1425,13 +1457,22 @@ gx_status gx_get_offsets(const gx_handle *h, int *blofs, int *bwofs, int *acofs,
   return GX_OK;
 }
 
-static gx_status record(gx_handle *h, cudaStream_t st, int stage, bool start)
+// Starts or ends a span of a stage.  A span that starts where the last one
+// ended (adjacent: nothing enqueued between) shares its event.
+static gx_status record(gx_handle *h, cudaStream_t st, int stage, bool start, bool adjacent)
 {
-  cudaEvent_t e;
-  CKR(h, cudaEventCreate(&e));
-  CKR(h, cudaEventRecord(e, st));
-  h->evs.push_back(e);
-  if (start) h->ev_stage.push_back(stage);
+  int e = h->nev - 1;
+  if (!(start && adjacent && e >= 0)) {
+    e = h->nev++;
+    if (e == (int)h->evs.size()) {
+      cudaEvent_t ev;
+      CKR(h, cudaEventCreate(&ev));
+      h->evs.push_back(ev);
+    }
+    CKR(h, cudaEventRecord(h->evs[e], st));
+  }
+  if (start) h->spans.push_back({stage, e, -1});
+  else h->spans.back().end = e;
   return GX_OK;
 }
 
@@ -1594,9 +1635,8 @@ gx_status gx_enqueue_subint(gx_handle *h, float2 *dev_results, cudaStream_t st)
   const DevJob &J = h->J;
   const bool timed = !h->untimed;
   if (timed) {
-    for (auto e : h->evs) cudaEventDestroy(e);
-    h->evs.clear();
-    h->ev_stage.clear();
+    h->spans.clear();
+    h->nev = 0;
   }
   h->launches = 0;
   const int k = h->slot;
@@ -1624,15 +1664,15 @@ gx_status gx_enqueue_subint(gx_handle *h, float2 *dev_results, cudaStream_t st)
 
   const int nbl = d.nbaselines;
   float4 *acc4 = reinterpret_cast<float4 *>(h->d_acc);
-  auto mark = [&](int stage, bool start) -> gx_status { return timed ? record(h, st, stage, start) : GX_OK; };
+  auto mark = [&](int stage, bool start, bool adjacent = false) -> gx_status {
+    return timed ? record(h, st, stage, start, adjacent) : GX_OK;
+  };
   const int nzr = (int)h->zrows.size(), nzf = (int)h->zfreq.size();
   if (h->nbins > 0) {
     CKR(h, cudaMemsetAsync(h->d_accb, 0, sizeof(float2) * h->binents.size() * h->nbins * J.nchan, st));
     CKR(h, cudaMemsetAsync(h->d_wbins, 0, sizeof(float) * h->binitems.size() * h->nbins, st));
   }
   const int npairs = (int)h->pairs.size();
-  CKR(h, cudaMemsetAsync(h->d_wacc, 0, sizeof(float) * (d.nstations + npairs), st));
-  CKR(h, cudaMemsetAsync(h->d_err, 0, sizeof(int), st));
   const int npc = (int)h->pcal.size();
   if (npc)
     CKR(h, cudaMemsetAsync(h->d_pcalbins, 0, sizeof(float2) * (size_t)h->pcal_chunks * npc * h->pcal_maxbins, st));
@@ -1643,11 +1683,11 @@ gx_status gx_enqueue_subint(gx_handle *h, float2 *dev_results, cudaStream_t st)
   // (first: the X-steps store their sums instead of adding to the accumulators)
   auto pass = [&](int b0, int nb, bool first) -> gx_status {
     gx_status r;
-    if ((r = mark(0, true)) != GX_OK) return r;
+    if ((r = mark(0, true, b0 > 0 && h->cur_npc[k] == 1)) != GX_OK) return r;
     const PcalFuse pf{h->d_pcalbins, h->d_pcalfirst, h->pcal_fuse_bins, h->pcal_maxbins, npc, h->pcal_chunks};
     bool pcal_done = false;
     CKR(h, fstep_launch(J, h->d_st, h->maxnrf, S, b0, nb, h->nslots, h->d_spec, h->d_w, h->d_bp, st,
-                        npc && h->pcal_fuse_bins ? &pf : nullptr, &pcal_done));
+                        npc && h->pcal_fuse_bins ? &pf : nullptr, &pcal_done, b0 == 0 ? h->d_err : nullptr));
     if (h->kurt && (r = gx_kurtosis_pass(h, nb, st)) != GX_OK) return r;
     if (npc && !pcal_done) {
       CKR(h, pcal_bins_launch(J, S, h->d_bp, nb, h->d_pcal, h->d_pcalrot, npc, h->pcal_per_station, h->pcal_chunks,
@@ -1655,10 +1695,10 @@ gx_status gx_enqueue_subint(gx_handle *h, float2 *dev_results, cudaStream_t st)
       h->launches += 1;
     }
     if ((r = mark(0, false)) != GX_OK) return r;
-    if ((r = mark(1, true)) != GX_OK) return r;
+    if ((r = mark(1, true, true)) != GX_OK) return r;
     if (h->tc)
       CKR(h, xmac_tc_launch(h->d_spec, nb, J.nchan, h->nfmain, J.ninputs, h->ks, h->hilo, h->d_scale, acc4,
-                            first ? 0 : 1, h->d_err, st));
+                            first ? 0 : 1, h->tc_upper, h->d_err, st));
     else
       CKR(h, xmac_fp32_launch(h->d_spec, nb, J.nrows, J.ninputs, J.nchan, h->nfmain, h->ks, h->d_acc, first ? 0 : 1, h->d_err,
                               st, h->xvar));
@@ -1679,7 +1719,7 @@ gx_status gx_enqueue_subint(gx_handle *h, float2 *dev_results, cudaStream_t st)
                               st));
       h->launches += 2;
     }
-    CKR(h, weights_launch(h->d_w, nb, d.nstations, h->d_pairs, npairs, h->d_wacc, st));
+    CKR(h, weights_launch(h->d_w, nb, d.nstations, h->d_pairs, npairs, h->d_wacc, b0 > 0 ? 1 : 0, st));
     if ((r = mark(1, false)) != GX_OK) return r;
     h->launches += 3;
     return GX_OK;
@@ -1709,7 +1749,11 @@ gx_status gx_enqueue_subint(gx_handle *h, float2 *dev_results, cudaStream_t st)
       if ((r = pass(b0, std::min(h->chunk, J.blocks_per_send - b0), b0 == 0)) != GX_OK) return r;
   }
   if (h->kurt && (r = gx_kurtosis_end(h, st)) != GX_OK) return r;
-  if ((r = mark(2, true)) != GX_OK) return r;
+  auto clear = [&]() -> gx_status {   // what the finalise kernels leave unwritten
+    if (!h->covered) CKR(h, cudaMemsetAsync(fin, 0, sizeof(float2) * h->rl_full, st));
+    return GX_OK;
+  };
+  if ((r = mark(2, true, !h->kurt)) != GX_OK) return r;
   if (nph > 1) {
     // baseline and autocorrelation weights; the shift decorrelation factors
     CKR(h, finalise_launch(nullptr, 0, h->d_acc, h->ks, h->acc_slice, J.nchan, h->d_went, (int)h->wents.size(),
@@ -1718,7 +1762,7 @@ gx_status gx_enqueue_subint(gx_handle *h, float2 *dev_results, cudaStream_t st)
                               reinterpret_cast<float *>(fin), 2 * h->bsd_first, st));
     h->launches += 2;
   } else if (h->tc) {
-    CKR(h, cudaMemsetAsync(fin, 0, sizeof(float2) * h->rl_full, st));
+    if ((r = clear()) != GX_OK) return r;
     CKR(h, finalise_tc_launch(h->d_tcprods, h->d_tcrows, (int)h->tcrows.size(), acc4, h->nfmain, J.nchan,
                               J.ninputs, h->ks, fin, st));
     CKR(h, finalise_launch(nullptr, 0, h->d_acc, h->ks, h->acc_slice, J.nchan, h->d_went, (int)h->wents.size(),
@@ -1733,11 +1777,11 @@ gx_status gx_enqueue_subint(gx_handle *h, float2 *dev_results, cudaStream_t st)
                                   fin, st));
     h->launches += 1;
   } else {
-    CKR(h, cudaMemsetAsync(fin, 0, sizeof(float2) * h->rl_full, st));
+    if ((r = clear()) != GX_OK) return r;
     CKR(h, finalise_launch(h->d_prods, (int)h->prods.size(), h->d_acc, h->ks, h->acc_slice, J.nchan, h->d_went,
                            (int)h->wents.size(), h->d_wacc, fin, st));
   }
-  if (nph == 1) h->launches += (h->prods.empty() ? 0 : 1) + (h->wents.empty() ? 0 : 1);
+  if (nph == 1) h->launches += h->tc ? (h->tcrows.empty() ? 0 : 1) + (h->wents.empty() ? 0 : 1) : 1;
   if (!h->zprods.empty()) {
     CKR(h, finalise_launch(h->d_zprods, (int)h->zprods.size(), h->d_accz, h->zks, h->zacc_slice, h->nzchan, nullptr,
                            0, nullptr, fin, st));
@@ -1892,12 +1936,12 @@ gx_status gx_stage_times(gx_handle *h, float ms[3])
 {
   if (!h || !ms) return GX_ERR_ARG;
   ms[0] = ms[1] = ms[2] = 0.f;
-  for (size_t i = 0; i + 1 < h->evs.size(); i += 2) {
-    CKR(h, cudaEventSynchronize(h->evs[i + 1]));
+  for (const gx_handle::Span &s : h->spans) {
+    if (s.end < 0) continue;
+    CKR(h, cudaEventSynchronize(h->evs[s.end]));
     float t = 0;
-    CKR(h, cudaEventElapsedTime(&t, h->evs[i], h->evs[i + 1]));
-    int stg = h->ev_stage[i / 2];
-    if (stg >= 0 && stg < 3) ms[stg] += t;
+    CKR(h, cudaEventElapsedTime(&t, h->evs[s.start], h->evs[s.end]));
+    if (s.stage >= 0 && s.stage < 3) ms[s.stage] += t;
   }
   return GX_OK;
 }

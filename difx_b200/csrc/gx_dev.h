@@ -60,6 +60,7 @@ struct DevJob {
   double inv_fftlen, inv_nchan;   // 1 / fftlen, 1 / nchan (powers of two: exact)
   const float2 *twiddle;  // exp(-2 pi i m / F), m in [0, F), then the pass rows of r16::tw_pass_offset
   float lut[256];         // level of each sample code (VDIF decode table), staged to shared memory
+  int lut_zero;           // some code's level is zero
   double lut_offset, lut_div;   // 8-bit codes: level = (code - lut_offset) / lut_div
   // 8-bit codes by arithmetic: level = fma(x, lut_hi, x * lut_lo) with
   // x = float(2^23 + code) - lut_bias; set only when the host has checked that

@@ -111,9 +111,11 @@ __device__ __forceinline__ int frame_ok(const uint8_t *frame, int framebytes, in
 
 // --------------------------------------------------------------------------
 // Per-block parameters (FP64): mode.cpp:656-757 and 782-799, mk5mode.cpp:94-174.
-__global__ void blockparams_kernel(DevJob J, SubintArrays S, int blk0, int nblk, BlockParam *__restrict__ bp,
-                                   float *__restrict__ weights)
+// The subint's first launch also clears the kernels' status (*clear_err, if given).
+__global__ void blockparams_kernel(const __grid_constant__ DevJob J, SubintArrays S, int blk0, int nblk,
+                                   BlockParam *__restrict__ bp, float *__restrict__ weights, int *clear_err)
 {
+  if (clear_err && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *clear_err = 0;
   const int bi = blockIdx.x * blockDim.x + threadIdx.x;
   const int s = blockIdx.y;
   if (bi >= nblk) return;
@@ -993,12 +995,12 @@ cudaError_t smem_opt_in(const void *kernel, size_t bytes)
 
 cudaError_t fstep_launch(const DevJob &J, const DevStation *stations, int maxnrf, const SubintArrays &S,
                          int blk0, int nblk, int nslots, float2 *spec, float *weights, BlockParam *bp,
-                         cudaStream_t st, const PcalFuse *pf, bool *pcal_done)
+                         cudaStream_t st, const PcalFuse *pf, bool *pcal_done, int *clear_err)
 {
   if (pcal_done) *pcal_done = false;
   {
     dim3 grid((nblk + 127) / 128, J.nstations);
-    blockparams_kernel<<<grid, 128, 0, st>>>(J, S, blk0, nblk, bp, weights);
+    blockparams_kernel<<<grid, 128, 0, st>>>(J, S, blk0, nblk, bp, weights, clear_err);
   }
   if (S.bandmask) {   // INTERLACEDVDIF: EDV4 per-band validity, one warp per (station, block)
     dim3 grid((nblk + 7) / 8, J.nstations);

@@ -98,6 +98,8 @@ struct gx_handle {
   std::vector<gx::ProdEntry> prods;
   std::vector<gx::TcProdEntry> tcprods;   // sorted by (freq, a)
   std::vector<gx::TcRowEntry> tcrows;
+  bool tc_upper = false;           // every tcprods entry lies on or above the diagonal (in 8 x 8 tiles)
+  bool covered = false;            // the finalise kernels write all of the full result array (no clearing before them)
   std::vector<gx::WeightEntry> wents;
   std::vector<int2> pairs;
   int xstep = 0;                   // X-step form in use (GX_XSTEP_AUTO resolved at open)
@@ -151,8 +153,14 @@ struct gx_handle {
 
   gx::SubintArrays last{};
   bool have_last = false;
-  std::vector<cudaEvent_t> evs;  // pairs per launch: [start, end]
-  std::vector<int> ev_stage;
+  // Stage timing: events kept from subint to subint; each span of a stage runs
+  // from one to another of this subint's (neighbouring spans share one).
+  struct Span {
+    int stage, start, end;
+  };
+  std::vector<cudaEvent_t> evs;
+  std::vector<Span> spans;
+  int nev = 0;                   // events recorded for this subint
   int launches = 0;
 
   std::vector<int> sta_acoff, sta_acw;   // [station * GX_MAX_BANDS + recorded band]: autocorrelation record, weight (-1: none)

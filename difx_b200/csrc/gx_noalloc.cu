@@ -229,7 +229,7 @@ extern "C" gx_status gx_subint_device_noalloc(const gx_job_desc *desc, const gx_
     const int nb = std::min(chunk, J.blocks_per_send - b0);
     NA_CK(fstep_launch(J, d_st, plan.maxnrf, S, b0, nb, plan.nslots, d_spec, d_w, d_bp, st));
     NA_CK(xmac_fp32_launch(d_spec, nb, J.nrows, J.ninputs, J.nchan, J.nfreqs, ks, d_acc, b0 > 0 ? 1 : 0, nullptr, st));
-    NA_CK(weights_launch(d_w, nb, nst, d_pairs, nbl, d_wacc, st));
+    NA_CK(weights_launch(d_w, nb, nst, d_pairs, nbl, d_wacc, 1, st));
   }
   NA_CK(finalise_launch(d_prods, (int)plan.prods.size(), d_acc, ks, acc_slice, J.nchan, d_went,
                         (int)plan.wents.size(), d_wacc, reinterpret_cast<float2 *>(dev_results), st));

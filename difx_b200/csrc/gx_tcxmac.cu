@@ -187,7 +187,8 @@ constexpr int kNumBars = 2 * kMaxStages + 2 * kOpStages + 1;   // full, empty, o
 template <bool HILO, int RP, int CW>
 __global__ void __launch_bounds__(tc_threads(CW), 1)
 xmac_tc_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int NP, int nfreqs, int ks, int ninputs,
-               const float *__restrict__ scale, float4 *__restrict__ acc, int accumulate, int *__restrict__ err)
+               const float *__restrict__ scale, float4 *__restrict__ acc, int accumulate, int upper,
+               int *__restrict__ err)
 {
   constexpr int kStages = TcRing<HILO, RP>::kStages;
   constexpr uint32_t kStageBytes = TcRing<HILO, RP>::kStageBytes;
@@ -435,7 +436,8 @@ xmac_tc_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int NP, i
         for (int m = 0; m < kNI * kVCols / kConvThreads; m++) {
           const int i = ct + kConvThreads * m;
           const int row = i / kVCols, col = i % kVCols;
-          if (row >= ninputs) continue;
+          // upper: nobody reads the 8 x 8 tiles below the diagonal
+          if (row >= ninputs || (upper && row / kVCols > cb)) continue;
           float4 w = sV[row * kVRow + col];
           float4 *dst = oblk + (size_t)row * kNI + cb * kVCols + col;
           if (accumulate) {
@@ -460,43 +462,55 @@ xmac_tc_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int NP, i
 // channel pairs stage acc[z][freq][p][a][bmin..127] (contiguous, summed over
 // the K-split slices) in shared memory, then every entry (a, b) of the row
 // writes its 2 kFinPairs channels as one contiguous run of the result array.
+//
+// What bounds it: HBM (64 stations, 4096 channels: 1.1 GB of accumulators and
+// 1.1 GB of results).  A warp takes whole rows of both phases: no index
+// divisions, and the staged rows have one pad element, because a warp's 32
+// channels of one entry lie a row apart (unpadded they were 16 deep in one
+// bank): with nothing cleared first, 1.06 -> 0.50 ms.
 constexpr int kFinPairs = 16;
+constexpr int kFinRow = kNI + 1;
 
 __global__ void __launch_bounds__(256)
 finalise_tc_kernel(const TcProdEntry *__restrict__ prods, const TcRowEntry *__restrict__ rows,
                    const float4 *__restrict__ acc, int nfreqs, int NP, int ks, int ninputs,
                    float2 *__restrict__ results)
 {
-  __shared__ float4 sV[kFinPairs][kNI];
+  __shared__ float4 sV[kFinPairs * kFinRow];
   const TcRowEntry R = rows[blockIdx.x];
   const size_t slice = (size_t)nfreqs * NP * kNI * kNI;
-  const int nb = ninputs - R.bmin;
-  const int ne = R.end - R.start;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // channel pairs [pb, pe) of this CTA (blockIdx.y of gridDim.y slices)
   const int per = ((NP + gridDim.y - 1) / gridDim.y + kFinPairs - 1) / kFinPairs * kFinPairs;
   const int pb = blockIdx.y * per, pe = min(NP, pb + per);
   for (int p0 = pb; p0 < pe; p0 += kFinPairs) {
     const int np = min(kFinPairs, pe - p0);
-    for (int i = threadIdx.x; i < np * nb; i += blockDim.x) {
-      const int pp = i / nb, b = R.bmin + i % nb;
-      const size_t off = (((size_t)R.freq * NP + p0 + pp) * kNI + R.a) * kNI + b;
-      float4 v = acc[off];
-      for (int z = 1; z < ks; z++) {
-        const float4 u = acc[z * slice + off];
-        v.x += u.x;
-        v.y += u.y;
-        v.z += u.z;
-        v.w += u.w;
+#pragma unroll
+    for (int m = 0; m < kFinPairs / 8; m++) {
+      const int pp = warp + 8 * m;
+      if (pp >= np) continue;
+      const float4 *row = acc + (((size_t)R.freq * NP + p0 + pp) * kNI + R.a) * kNI;
+#pragma unroll
+      for (int i = 0; i < kNI / 32; i++) {
+        const int b = R.bmin + lane + 32 * i;
+        if (b >= ninputs) continue;
+        float4 v = row[b];
+        for (int z = 1; z < ks; z++) {
+          const float4 u = row[z * slice + b];
+          v.x += u.x;
+          v.y += u.y;
+          v.z += u.z;
+          v.w += u.w;
+        }
+        sV[pp * kFinRow + b] = v;
       }
-      sV[pp][b] = v;
     }
     __syncthreads();
-    const int nc = 2 * np;
-    for (int i = threadIdx.x; i < ne * nc; i += blockDim.x) {
-      const TcProdEntry P = prods[R.start + i / nc];
-      const int cc = i % nc;
-      const float4 v = sV[cc >> 1][P.b];
-      results[P.result_offset + 2 * p0 + cc] = (cc & 1) ? make_float2(v.z, v.w) : make_float2(v.x, v.y);
+    if (lane < 2 * np) {
+      const float2 *v = reinterpret_cast<const float2 *>(sV + (lane >> 1) * kFinRow) + (lane & 1);
+      float2 *dst = results + 2 * p0 + lane;
+#pragma unroll 4
+      for (int e = R.start + warp; e < R.end; e += 8) dst[prods[e].result_offset] = v[2 * prods[e].b];
     }
     __syncthreads();
   }
@@ -548,7 +562,7 @@ size_t xmac_tc_smem_bytes(bool hilo)
 }
 
 cudaError_t xmac_tc_launch(const float2 *spec, int nblk, int N, int nfreqs, int ninputs, int ks, bool hilo,
-                           const float *scale, float4 *acc, int accumulate, int *err, cudaStream_t st)
+                           const float *scale, float4 *acc, int accumulate, bool upper, int *err, cudaStream_t st)
 {
   if (nblk <= 0) return cudaSuccess;
   if (ninputs < 1 || ninputs > kNI) return cudaErrorInvalidValue;
@@ -574,7 +588,7 @@ cudaError_t xmac_tc_launch(const float2 *spec, int nblk, int N, int nfreqs, int 
     cudaError_t e = smem_opt_in((const void *)xmac_tc_kernel<H, RPV, CWV>, sm);                             \
     if (e != cudaSuccess) return e;                                                                         \
     xmac_tc_kernel<H, RPV, CWV><<<grid, tc_threads(CWV), sm, st>>>(map, nblk, N / 2, nfreqs, ks, ninputs,   \
-                                                                    scale, acc, accumulate, err);           \
+                                                                    scale, acc, accumulate, upper ? 1 : 0, err); \
     return cudaGetLastError();                                                                              \
   }
   GX_TC_CASE(true, 1, 16) GX_TC_CASE(false, 1, 16) GX_TC_CASE(true, 1, 8) GX_TC_CASE(false, 1, 8)

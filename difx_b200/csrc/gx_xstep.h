@@ -52,10 +52,12 @@ cudaError_t fstep_pair_launch(const DevJob &J, const DevStation *stations, const
                               const BlockParam *bp, float2 *spec, cudaStream_t st, const PcalFuse *pf, bool *pcal_done);
 // F-step of one pass of blocks.  With pf, the paired-band kernel also forms
 // the phase-cal bin sums when it takes the job; *pcal_done (if given) tells
-// whether it did (else the caller runs pcal_bins_launch).
+// whether it did (else the caller runs pcal_bins_launch).  clear_err: a status
+// word to clear first.
 cudaError_t fstep_launch(const DevJob &J, const DevStation *stations, int maxnrf, const SubintArrays &S,
                          int blk0, int nblk, int nslots, float2 *spec, float *weights, BlockParam *bp,
-                         cudaStream_t st, const PcalFuse *pf = nullptr, bool *pcal_done = nullptr);
+                         cudaStream_t st, const PcalFuse *pf = nullptr, bool *pcal_done = nullptr,
+                         int *clear_err = nullptr);
 // FP32 X-step over one pass of blocks, NI spectra rows of which the first
 // `rows` are in use; accumulate 0: acc is overwritten (its upper tiles), not
 // added to.  *err (may be null) receives a nonzero status if a wait of the
@@ -65,8 +67,9 @@ cudaError_t fstep_launch(const DevJob &J, const DevStation *stations, int maxnrf
 constexpr int kXmacVariants = 2;
 cudaError_t xmac_fp32_launch(const float2 *spec, int nblk, int rows, int NI, int N, int nfreqs, int ks, float2 *acc,
                              int accumulate, int *err, cudaStream_t st, int variant = 0);
+// Weight sums of one pass of blocks; accumulate 0: wacc is overwritten.
 cudaError_t weights_launch(const float *w, int nblk, int nstations, const int2 *pairs, int npairs, float *wacc,
-                           cudaStream_t st);
+                           int accumulate, cudaStream_t st);
 // Entries [start, end) of the tensor-core product table (sorted by freq, then a)
 // share row a of freq; bmin is their smallest b.
 struct TcRowEntry {
@@ -76,10 +79,11 @@ struct TcRowEntry {
 // Tensor-core X-step over spectra [freq][block][ninputs][N] (ninputs <= 128,
 // the MMA tile's M; missing rows are zeros); acc holds, per K-split slice,
 // [freq][N/2][128][128] float4 = (Re, Im) of both channels of a channel pair,
-// unscaled, of which rows and columns below ninputs are written.
+// unscaled, of which rows and columns below ninputs are written (upper: only
+// the 8 x 8 tiles on and above the diagonal).
 size_t xmac_tc_smem_bytes(bool hilo);
 cudaError_t xmac_tc_launch(const float2 *spec, int nblk, int N, int nfreqs, int ninputs, int ks, bool hilo,
-                           const float *scale, float4 *acc, int accumulate, int *err, cudaStream_t st);
+                           const float *scale, float4 *acc, int accumulate, bool upper, int *err, cudaStream_t st);
 cudaError_t finalise_tc_launch(const TcProdEntry *prods, const TcRowEntry *rows, int nrows, const float4 *acc,
                                int nfreqs, int N, int ninputs, int ks, float2 *results, cudaStream_t st);
 // One record of channel averaging (CHANS TO AVG): n output values at dst, each
