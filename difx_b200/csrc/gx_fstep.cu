@@ -271,7 +271,17 @@ __global__ void edv4_kernel(DevJob J, const DevStation *__restrict__ stations, S
         }
       }
       // count the non-zero samples the masks blank (decoder-valid frames only)
-      for (int b = 0; b < nb; b++) {
+      if (!J.lut_zero) {
+        // no level is zero: every sample of the blanked frames counts, no need
+        // to read them (6 stations, 3126 blocks, 5 % partial frames: 50 -> 8 us)
+        for (unsigned long long m = lane < nb ? mymask & P.validmask : 0ull; m; m &= m - 1) {
+          const long long fr = (long long)P.fr0 + (__ffsll(m) - 1);
+          const long long lo = max((long long)P.nearestsample, fr * fs);
+          const long long hi = min((long long)P.nearestsample + J.fftlen, (fr + 1) * fs);
+          inv += (int)max(hi - lo, 0ll);
+        }
+      }
+      for (int b = 0; J.lut_zero && b < nb; b++) {
         const unsigned long long bmask = __shfl_sync(0xffffffffu, mymask, b) & P.validmask;
         if (!bmask) continue;
         int cnt = 0;
@@ -879,17 +889,20 @@ __global__ void __launch_bounds__(256) pcal_station_kernel(DevJob J, SubintArray
 }
 
 // Tone t of band pb: the forward DFT of the bins at bin offset_bin + t step,
-// summed in double and rounded once (the reference's DFT of its bins).
-__global__ void __launch_bounds__(128) pcal_tones_kernel(const PcalBand *__restrict__ bands, int chunks, int maxbins,
+// summed in double and rounded once (the reference's DFT of its bins).  A warp
+// per tone, its lanes over the bins (a thread per tone went through the bins one
+// FP64 sincos after the other: 32 bands of 16 tones, 19 -> 7 us).
+__global__ void __launch_bounds__(256) pcal_tones_kernel(const PcalBand *__restrict__ bands, int chunks, int maxbins,
                                                          const float2 *__restrict__ partial, float2 *__restrict__ results)
 {
   const int pb = blockIdx.x;
   const PcalBand B = bands[pb];
-  for (int t = threadIdx.x; t < B.ntones; t += blockDim.x) {
+  const int lane = threadIdx.x & 31;
+  for (int t = threadIdx.x >> 5; t < B.ntones; t += blockDim.x >> 5) {
     const long long bin = (long long)B.offset_bin + (long long)t * B.step;
     double re = 0.0, im = 0.0;
     if (B.nbins > 0 && bin < B.nbins && t < B.nextract) {
-      for (int k = 0; k < B.nbins; k++) {
+      for (int k = lane; k < B.nbins; k += 32) {
         float bx = 0.f, by = 0.f;   // the bin, summed over the chunks in order
         for (int c = 0; c < chunks; c++) {
           const float2 v = partial[((size_t)c * gridDim.x + pb) * maxbins + k];
@@ -902,8 +915,12 @@ __global__ void __launch_bounds__(128) pcal_tones_kernel(const PcalBand *__restr
         re += (double)bx * cs - (double)by * sn;
         im += (double)bx * sn + (double)by * cs;
       }
+      for (int o = 16; o > 0; o >>= 1) {
+        re += __shfl_xor_sync(0xffffffffu, re, o);
+        im += __shfl_xor_sync(0xffffffffu, im, o);
+      }
     }
-    results[B.result_offset + t] = make_float2((float)re, (float)im);
+    if (lane == 0) results[B.result_offset + t] = make_float2((float)re, (float)im);
   }
 }
 
@@ -945,27 +962,40 @@ cudaError_t pcal_bins_launch(const DevJob &J, const SubintArrays &S, const Block
   return cudaGetLastError();
 }
 
-// Sum of the chunks' partial bin sums into chunk 0, in chunk order (the order
-// the tones kernel would add them in): one thread per (band, bin), loads
-// coalesced across threads.
+// Sum of the chunks' partial bin sums into chunk 0: 32 (band, bin) sums a CTA,
+// the chunks in eight runs summed side by side and then in order, so that the
+// sums do not depend on timing (one thread a sum took the chunks one after the
+// other: 1024 sums of 391 chunks, 59 -> 9 us).
 __global__ void __launch_bounds__(256) pcal_fold_kernel(float2 *__restrict__ partial, int chunks, long long n)
 {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  __shared__ float2 s_run[8][32];
+  const int lane = threadIdx.x & 31, run = threadIdx.x >> 5;
+  const long long i = (long long)blockIdx.x * 32 + lane;
+  const int per = (chunks + 7) / 8, c1 = min(chunks, (run + 1) * per);
   float bx = 0.f, by = 0.f;
+  if (i < n) {
 #pragma unroll 8
-  for (int c = 0; c < chunks; c++) {
-    const float2 v = partial[(size_t)c * n + i];
-    bx += v.x;
-    by += v.y;
+    for (int c = run * per; c < c1; c++) {
+      const float2 v = partial[(size_t)c * n + i];
+      bx += v.x;
+      by += v.y;
+    }
   }
-  partial[i] = make_float2(bx, by);
+  s_run[run][lane] = make_float2(bx, by);
+  __syncthreads();
+  if (run == 0 && i < n) {
+    for (int r = 1; r < 8; r++) {
+      bx += s_run[r][lane].x;
+      by += s_run[r][lane].y;
+    }
+    partial[i] = make_float2(bx, by);
+  }
 }
 
 cudaError_t pcal_fold_launch(float2 *partial, int chunks, long long n, cudaStream_t st)
 {
   if (chunks <= 1 || n <= 0) return cudaSuccess;
-  pcal_fold_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(partial, chunks, n);
+  pcal_fold_kernel<<<(unsigned)((n + 31) / 32), 256, 0, st>>>(partial, chunks, n);
   return cudaGetLastError();
 }
 
@@ -973,7 +1003,7 @@ cudaError_t pcal_tones_launch(const PcalBand *bands, int nbands, int chunks, int
                               float2 *results, cudaStream_t st)
 {
   if (nbands <= 0) return cudaSuccess;
-  pcal_tones_kernel<<<nbands, 128, 0, st>>>(bands, chunks, maxbins, partial, results);
+  pcal_tones_kernel<<<nbands, 256, 0, st>>>(bands, chunks, maxbins, partial, results);
   return cudaGetLastError();
 }
 
