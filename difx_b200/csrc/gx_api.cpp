@@ -895,6 +895,13 @@ static gx_status setup(gx_handle *h)
         }
     }
   }
+  h->paired_ok = h->tc && J.pair_same && J.nbands % 2 == 0 && J.ninputs % 2 == 0 && h->zfreq.empty() &&
+                 fstep_pair_eligible(J);
+  for (int s = 0; s < d.nstations; s++)
+    for (int b = 0; b + 1 < d.stations[s].nbands; b += 2) {
+      const int r = h->band_input[s][b];
+      h->paired_ok = h->paired_ok && r % 2 == 0 && h->band_input[s][b + 1] == r + 1;
+    }
   h->tc_upper = true;
   for (const TcProdEntry &t : h->tcprods) h->tc_upper = h->tc_upper && t.b / 8 >= t.a / 8;
 
@@ -1632,7 +1639,10 @@ static gx_status stage_subint(gx_handle *h, const gx_subint_desc *sub, const uin
 gx_status gx_enqueue_subint(gx_handle *h, float2 *dev_results, cudaStream_t st)
 {
   const gx_job_desc &d = h->jd;
-  const DevJob &J = h->J;
+  // pairs of rows interleaved where only the F-step and the tensor-core X-step
+  // see the spectra
+  DevJob J = h->J;
+  J.paired = h->paired_ok && !h->kurt ? 1 : 0;
   const bool timed = !h->untimed;
   if (timed) {
     h->spans.clear();
@@ -1697,7 +1707,7 @@ gx_status gx_enqueue_subint(gx_handle *h, float2 *dev_results, cudaStream_t st)
     if ((r = mark(0, false)) != GX_OK) return r;
     if ((r = mark(1, true, true)) != GX_OK) return r;
     if (h->tc)
-      CKR(h, xmac_tc_launch(h->d_spec, nb, J.nchan, h->nfmain, J.ninputs, h->ks, h->hilo, h->d_scale, acc4,
+      CKR(h, xmac_tc_launch(h->d_spec, nb, J.nchan, h->nfmain, J.ninputs, J.paired != 0, h->ks, h->hilo, h->d_scale, acc4,
                             first ? 0 : 1, h->tc_upper, h->d_err, st));
     else
       CKR(h, xmac_fp32_launch(h->d_spec, nb, J.nrows, J.ninputs, J.nchan, h->nfmain, h->ks, h->d_acc, first ? 0 : 1, h->d_err,

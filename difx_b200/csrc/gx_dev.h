@@ -54,6 +54,7 @@ struct DevJob {
   int lgstride;           // log2(stride): FFT length, channels and stride are powers of two
   int fringe_order;       // FRINGE ROTN ORDER: 1 pre-F linear, 2 pre-F quadratic, 0 post-F (real data)
   int deltapol_any;       // some station has a second (polarisation B) fractional-sample rotator
+  int paired;             // spectra rows 2s and 2s + 1 interleaved by channel: [freq][block][row pair][channel][2]
   int pair_same;          // bands 2p and 2p + 1 share local freq and fractional-sample rotator at every station
   double sampletime;      // us
   double bw;              // MHz

@@ -805,45 +805,64 @@ fstep_pair_kernel(const __grid_constant__ DevJob J, const DevStation *__restrict
         // the thread's steps: consecutive, from register 0's channel on (a split
         // group's upper eight registers are 16 steps on)
         const int s0 = (jj >> LGS) * (N / C::NTS) + (C::SPLIT ? 8 * h : 0);
-        auto corr = [&](const float4 *fpj, float2 fsk, int t) {
-          const float4 q = fpj[(C::SPLIT && t >= 8 ? t + 8 : t) / 2];
-          return cmul(fsk, t & 1 ? make_float2(q.z, q.w) : make_float2(q.x, q.y));
+        // register t's channel and whether its value is conjugated (complex lower sideband)
+        auto channel = [&](int t, int lsb, bool &conj) {
+          const int bin = c0 + hop(t);
+          conj = CPLX && lsb && bin != 0;
+          return conj ? F - bin : bin;
         };
-        auto emit = [&](int lane, const float2 *tab, int bd, int lf, int lsb) {
+        // its correction from a band's tables
+        auto corr = [&](const float2 *tab, int lsb, int t) {
           const float2 *fs = tab + SD + C::NFR, *fp = fs + SD;
-          float2 *row = spec + (((size_t)st.freq_index[lf] * nblk + bi) * J.ninputs + st.band_input[bd]) * N;
           if (CPLX && lsb) {
-            const float2 fsk = fs[(-jj) & (SD - 1)];
-#pragma unroll
-            for (int t = 0; t < 16; t++) {
-              const int bin = c0 + hop(t), c = bin == 0 ? 0 : F - bin;
-              float2 val = pick(t, lane);
-              if (bin != 0) val.y = -val.y;
-              row[c] = cmul(val, cmul(fsk, fp[step_pos<C::NTS, SD>(c >> LGS, N / C::NTS)]));
-            }
-          } else {
-            const float2 fsk = fs[jj & (SD - 1)];
-            const float4 *fpj = reinterpret_cast<const float4 *>(fp + s0);
-            row += c0;
-#pragma unroll
-            for (int t = 0; t < NOUT; t++) row[hop(t)] = cmul(pick(t, lane), corr(fpj, fsk, t));
+            bool conj;
+            const int c = channel(t, lsb, conj);
+            return cmul(fs[(-jj) & (SD - 1)], fp[step_pos<C::NTS, SD>(c >> LGS, N / C::NTS)]);
           }
+          const float4 q = reinterpret_cast<const float4 *>(fp + s0)[(C::SPLIT && t >= 8 ? t + 8 : t) / 2];
+          return cmul(fs[jj & (SD - 1)], t & 1 ? make_float2(q.z, q.w) : make_float2(q.x, q.y));
         };
-        if (SAME && !(CPLX && lsb0)) {
+        auto value = [&](int t, int lane, bool conj) {
+          float2 val = pick(t, lane);
+          if (conj) val.y = -val.y;
+          return val;
+        };
+        if (SAME) {
           // both bands by the same correction
-          const float2 *fs = tab0 + SD + C::NFR;
-          const float4 *fpj = reinterpret_cast<const float4 *>(fs + SD + s0);
-          const float2 fsk = fs[jj & (SD - 1)];
           const size_t base = ((size_t)st.freq_index[lf0] * nblk + bi) * J.ninputs;
-          float2 *row0 = spec + (base + st.band_input[bd0]) * N + c0;
-          float2 *row1 = spec + (base + st.band_input[bd1]) * N + c0;
+          float2 *row0 = spec + (base + st.band_input[bd0]) * N;
+          float2 *row1 = spec + (base + st.band_input[bd1]) * N;
+          auto both = [&](int lsb, bool paired) {
 #pragma unroll
-          for (int t = 0; t < NOUT; t++) {
-            const float2 w = corr(fpj, fsk, t);
-            row0[hop(t)] = cmul(pick(t, 0), w);
-            if (has1) row1[hop(t)] = cmul(pick(t, 1), w);
-          }
+            for (int t = 0; t < NOUT; t++) {
+              bool conj;
+              const int c = channel(t, lsb, conj);
+              const float2 w = corr(tab0, lsb, t);
+              const float2 x = cmul(value(t, 0, conj), w), y = cmul(value(t, 1, conj), w);
+              if (paired) {
+                reinterpret_cast<float4 *>(row0)[c] = make_float4(x.x, x.y, y.x, y.y);
+              } else {
+                row0[c] = x;
+                if (has1) row1[c] = y;
+              }
+            }
+          };
+          if (CPLX && lsb0) J.paired ? both(1, true) : both(1, false);
+          else J.paired ? both(0, true) : both(0, false);
         } else {
+          auto one = [&](int lane, const float2 *tab, int bd, int lf, int lsb) {
+            float2 *row = spec + (((size_t)st.freq_index[lf] * nblk + bi) * J.ninputs + st.band_input[bd]) * N;
+#pragma unroll
+            for (int t = 0; t < NOUT; t++) {
+              bool conj;
+              const int c = channel(t, lsb, conj);
+              row[c] = cmul(value(t, lane, conj), corr(tab, lsb, t));
+            }
+          };
+          auto emit = [&](int lane, const float2 *tab, int bd, int lf, int lsb) {
+            if (CPLX && lsb) one(lane, tab, bd, lf, 1);
+            else one(lane, tab, bd, lf, 0);
+          };
           emit(0, tab0, bd0, lf0, lsb0);
           if (has1) emit(1, tab1, bd1, lf1, lsb1);
         }

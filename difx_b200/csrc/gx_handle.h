@@ -98,6 +98,7 @@ struct gx_handle {
   std::vector<gx::ProdEntry> prods;
   std::vector<gx::TcProdEntry> tcprods;   // sorted by (freq, a)
   std::vector<gx::TcRowEntry> tcrows;
+  bool paired_ok = false;          // the bands of a pair are rows 2s, 2s + 1 everywhere: spectra may be paired
   bool tc_upper = false;           // every tcprods entry lies on or above the diagonal (in 8 x 8 tiles)
   bool covered = false;            // the finalise kernels write all of the full result array (no clearing before them)
   std::vector<gx::WeightEntry> wents;

@@ -19,7 +19,7 @@
 // Data path per CTA: the spectra spec[freq][block][input][chan] (float2, as the
 // F-step writes them) are read as a 4-D FP32 tensor; one TMA tile load (no
 // multicast) per 16 blocks fetches the 4 floats of the CTA's channel pair for
-// all 128 inputs ([block][input][16 bytes], blocks past the chunk and rows
+// all 128 inputs ([block][input][16 bytes], or two inputs to a 32-byte row, blocks past the chunk and rows
 // past the job's inputs read as zeros) into a 4-stage FP32 ring.  The CTA's
 // warps have roles joined only by mbarriers: one lane of warp 0 issues the
 // tile loads as stages free up; eight converter warps scale each value by a
@@ -66,15 +66,12 @@ constexpr uint32_t kXrOffset = (kNI / 8) * kSBO;          // rows 128.. (Xr) sta
 constexpr int kPRow = kNI + 1;               // padded row of the P matrices parked in shared memory
 constexpr int kVCols = 8;                    // columns of V per epilogue slice (one 128-byte line per row)
 constexpr int kVRow = kVCols + 1;            // padded slice row, float4
-// FP32 staging ring: RP channel pairs per tile row (RP = 2: whole 32-byte
-// sectors, half the row requests of RP = 1), as many stages as fit beside the
-// operand stages.
-template <bool HILO, int RP>
+constexpr int kRingStages = 4;               // FP32 staging ring
+constexpr uint32_t kStageBytes = kKT * kRowBytes;   // 32 KB
+template <bool HILO>
 struct TcRing {
-  static constexpr uint32_t kStageBytes = kKT * kRowBytes * RP;   // 32 or 64 KB
-  static constexpr int kStages = RP == 1 ? 4 : (HILO ? 2 : 3);
   static constexpr uint32_t kOpStageBytes = (HILO ? 2 : 1) * 2 * kOpChanBytes;
-  static_assert((2 * kNI * kPRow + 2 * kNI) * 4 + kNI * kVRow * 16 <= kStages * kStageBytes + kOpStages * kOpStageBytes,
+  static_assert((2 * kNI * kPRow + 2 * kNI) * 4 + kNI * kVRow * 16 <= kRingStages * kStageBytes + kOpStages * kOpStageBytes,
                 "epilogue tables must fit in the staging ring and operand stages");
 };
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -179,25 +176,28 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t &hi, uint32_t 
 // of its neighbours.
 constexpr int kConvThreads = 256;            // converter threads that also run the epilogue
 constexpr int kConvWarp0 = 2;
-// threads of a CTA with CW converter warps: 1 load warp, 1 MMA warp, CW converters
-__host__ __device__ constexpr int tc_threads(int cw) { return 32 * (kConvWarp0 + cw); }
-constexpr int kMaxStages = 4;
-constexpr int kNumBars = 2 * kMaxStages + 2 * kOpStages + 1;   // full, empty, opfull, opempty, done
+constexpr int kConvWarps = kConvThreads / 32;
+constexpr int kTcThreads = 32 * (kConvWarp0 + kConvWarps);   // 1 load warp, 1 MMA warp, the converters
+constexpr int kNumBars = 2 * kRingStages + 2 * kOpStages + 1;   // full, empty, opfull, opempty, done
 
-template <bool HILO, int RP, int CW>
-__global__ void __launch_bounds__(tc_threads(CW), 1)
+// PAIRED: rows of two inputs, [block][input pair][channel][2], as the
+// paired-band F-step writes the two polarisations of a station.  A tile is then
+// 1024 rows of 32 bytes instead of 2048 of 16: the tile loads bound the kernel, at
+// a rate of rows, and 16-byte rows move half-used sectors (64 stations, 4096
+// channels, 500 blocks: X stage 3.01 -> 2.58 ms split, 2.66 -> 1.93 ms single).
+template <bool HILO, bool PAIRED>
+__global__ void __launch_bounds__(kTcThreads, 1)
 xmac_tc_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int NP, int nfreqs, int ks, int ninputs,
                const float *__restrict__ scale, float4 *__restrict__ acc, int accumulate, int upper,
                int *__restrict__ err)
 {
-  constexpr int kStages = TcRing<HILO, RP>::kStages;
-  constexpr uint32_t kStageBytes = TcRing<HILO, RP>::kStageBytes;
-  constexpr uint32_t kOpStageBytes = TcRing<HILO, RP>::kOpStageBytes;
+  constexpr int kStages = kRingStages;
+  constexpr uint32_t kOpStageBytes = TcRing<HILO>::kOpStageBytes;
   extern __shared__ __align__(1024) unsigned char smem[];
   unsigned char *staging = smem;
   unsigned char *ops = smem + kStages * kStageBytes;
   uint64_t *bars = reinterpret_cast<uint64_t *>(ops + kOpStages * kOpStageBytes);
-  uint64_t *full = bars, *empty = bars + kMaxStages, *opfull = bars + 2 * kMaxStages;
+  uint64_t *full = bars, *empty = bars + kRingStages, *opfull = bars + 2 * kRingStages;
   uint64_t *opempty = opfull + kOpStages, *done = opempty + kOpStages;
   uint32_t *s_tmem = reinterpret_cast<uint32_t *>(bars + kNumBars);
   volatile int *s_abort = reinterpret_cast<volatile int *>(s_tmem + 1);
@@ -208,7 +208,7 @@ xmac_tc_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int NP, i
   const int ntile_all = (nblk + kKT - 1) / kKT;
   const int t0 = (int)((long long)ntile_all * z / ks);
   const int nt = (int)((long long)ntile_all * (z + 1) / ks) - t0;
-  const int nconv_warps = CW;
+  const int nconv_warps = kConvWarps;
 
   if (tid == 0) {
     for (int i = 0; i < kStages; i++) {
@@ -248,7 +248,7 @@ xmac_tc_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int NP, i
       }
       const uint32_t bar = smem_u32(full + st);
       mbar_expect_tx(bar, kStageBytes);
-      tma_load_4d(smem_u32(staging + st * kStageBytes), &spec_map, 4 * RP * (p / RP), 0, (t0 + u) * kKT, f, bar);
+      tma_load_4d(smem_u32(staging + st * kStageBytes), &spec_map, (PAIRED ? 8 : 4) * p, 0, (t0 + u) * kKT, f, bar);
       issued = u + 1;
     }
   } else if (warp == 1 && lane == 0) {
@@ -283,15 +283,23 @@ xmac_tc_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int NP, i
     }
     if (!*s_abort && mmas == nt && nt > 0) mma_commit(smem_u32(done));
   } else if (warp >= kConvWarp0) {
-    // ---- converters: row r, blocks k0 .. k0 + BPT - 1 of each tile
-    constexpr int BPT = 64 / CW;   // blocks per thread: 8 (8 warps) or 4 (16 warps)
-    constexpr int NW = BPT / 2;    // half2 words per quantity
+    // ---- converters: 16-byte piece r of each block of a tile, blocks k0 ..
+    // k0 + BPT - 1: both channels of input r, or (PAIRED) inputs r and r ^ 1 of
+    // channel r & 1, r itself first, so that the eight lanes of a 128-byte phase
+    // store to eight neighbouring rows
+    constexpr int BPT = 64 / kConvWarps;   // blocks per thread
+    constexpr int NW = BPT / 2;            // half2 words per quantity
     const int ct = tid - kConvWarp0 * 32;
     const int r = ct & (kNI - 1), k0 = (ct >> 7) * BPT;
-    const float s0 = scale[((size_t)f * kNI + r) * N + 2 * p];
-    const float s1 = scale[((size_t)f * kNI + r) * N + 2 * p + 1];
-    const uint32_t row_off = (uint32_t)(r >> 3) * kSBO + (uint32_t)(k0 >> 3) * kLBO + (uint32_t)(r & 7) * 16 +
-                             (uint32_t)(k0 & 7) * 2;
+    const int e0 = PAIRED ? (r & 1) : 0, e1 = PAIRED ? e0 : 1;   // channel and input of the first and second value
+    const int r1 = PAIRED ? r ^ 1 : r;
+    const float s0 = scale[((size_t)f * kNI + r) * N + 2 * p + e0];
+    const float s1 = scale[((size_t)f * kNI + r1) * N + 2 * p + e1];
+    auto place = [&](int row, int e) {
+      return (uint32_t)(row >> 3) * kSBO + (uint32_t)(k0 >> 3) * kLBO + (uint32_t)(row & 7) * 16 + (uint32_t)(k0 & 7) * 2 +
+             (uint32_t)e * kOpChanBytes;
+    };
+    const uint32_t at0 = place(r, e0), at1 = place(r1, e1);
     for (int t = 0; t < nt; t++) {
       if (*s_abort) break;
       const int st = t % kStages, o = t % kOpStages;
@@ -300,16 +308,18 @@ xmac_tc_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int NP, i
         break;
       }
       const int kv = min(kKT, nblk - (t0 + t) * kKT);
-      // row (k, r) of the stage holds RP channel pairs; this CTA's is pair p % RP
-      const float4 *stg = reinterpret_cast<const float4 *>(staging + st * kStageBytes) + (p % RP);
+      const float4 *stg = reinterpret_cast<const float4 *>(staging + st * kStageBytes);
+      // (value 0 re, im, value 1 re, im) at block k; of an odd piece of a pair, input r is the second
+      auto piece = [&](int k) {
+        const float4 x = (k < kv) ? stg[k * kNI + r] : make_float4(0.f, 0.f, 0.f, 0.f);
+        return PAIRED && e0 ? make_float4(x.z, x.w, x.x, x.y) : x;
+      };
       uint32_t re0[NW], im0[NW], re1[NW], im1[NW];
       uint32_t lre0[NW], lim0[NW], lre1[NW], lim1[NW];
 #pragma unroll
       for (int j = 0; j < NW; j++) {
         const int k = k0 + 2 * j;
-        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-        const float4 a = (k < kv) ? stg[(k * kNI + r) * RP] : zero;   // (c0.re, c0.im, c1.re, c1.im) at block k
-        const float4 b = (k + 1 < kv) ? stg[((k + 1) * kNI + r) * RP] : zero;
+        const float4 a = piece(k), b = piece(k + 1);
         if (HILO) {
           split2(a.x * s0, b.x * s0, re0[j], lre0[j]);
           split2(a.y * s0, b.y * s0, im0[j], lim0[j]);
@@ -334,16 +344,16 @@ xmac_tc_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int NP, i
         if constexpr (NW == 4) *reinterpret_cast<uint4 *>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
         else *reinterpret_cast<uint2 *>(dst) = make_uint2(w[0], w[1]);
       };
-      put(op + row_off, im0);
-      put(op + row_off + kXrOffset, re0);
-      put(op + kOpChanBytes + row_off, im1);
-      put(op + kOpChanBytes + row_off + kXrOffset, re1);
+      put(op + at0, im0);
+      put(op + at0 + kXrOffset, re0);
+      put(op + at1, im1);
+      put(op + at1 + kXrOffset, re1);
       if (HILO) {
         unsigned char *lo = op + 2 * kOpChanBytes;
-        put(lo + row_off, lim0);
-        put(lo + row_off + kXrOffset, lre0);
-        put(lo + kOpChanBytes + row_off, lim1);
-        put(lo + kOpChanBytes + row_off + kXrOffset, lre1);
+        put(lo + at0, lim0);
+        put(lo + at0 + kXrOffset, lre0);
+        put(lo + at1, lim1);
+        put(lo + at1 + kXrOffset, lre1);
       }
       fence_proxy_async_smem();
       __syncwarp();
@@ -543,58 +553,37 @@ cudaError_t tma_map_f32_4d(CUtensorMap *map, const void *base, const cuuint64_t 
   return cr == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-// Channel pairs per staged tile row: 1 (16-byte rows, four stages) unless
-// GX_TC_ROW_PAIRS=2 (32-byte rows, fewer stages; measured no faster on C3).
-static int tc_row_pairs()
-{
-  const char *e = getenv("GX_TC_ROW_PAIRS");
-  return (e && atoi(e) == 2) ? 2 : 1;
-}
-
 size_t xmac_tc_smem_bytes(bool hilo)
 {
-  const int rp = tc_row_pairs();
-  const size_t ring = rp == 1 ? (size_t)TcRing<true, 1>::kStages * TcRing<true, 1>::kStageBytes
-                              : (hilo ? (size_t)TcRing<true, 2>::kStages * TcRing<true, 2>::kStageBytes
-                                      : (size_t)TcRing<false, 2>::kStages * TcRing<false, 2>::kStageBytes);
-  const size_t ops = (size_t)kOpStages * (hilo ? 2 : 1) * 2 * kOpChanBytes;
-  return ring + ops + kNumBars * 8 + 16;
+  return (size_t)kRingStages * kStageBytes + (size_t)kOpStages * (hilo ? 2 : 1) * 2 * kOpChanBytes + kNumBars * 8 + 16;
 }
 
-cudaError_t xmac_tc_launch(const float2 *spec, int nblk, int N, int nfreqs, int ninputs, int ks, bool hilo,
+cudaError_t xmac_tc_launch(const float2 *spec, int nblk, int N, int nfreqs, int ninputs, bool paired, int ks, bool hilo,
                            const float *scale, float4 *acc, int accumulate, bool upper, int *err, cudaStream_t st)
 {
   if (nblk <= 0) return cudaSuccess;
-  if (ninputs < 1 || ninputs > kNI) return cudaErrorInvalidValue;
-  // spec[freq][block][row][channel] float2 as a 4-D FP32 tensor (innermost first):
-  // {2N floats, ninputs rows, nblk blocks, nfreqs}; box {4 floats, 128 rows, kKT
-  // blocks, 1}: the rows beyond the job's inputs (and blocks beyond nblk) are
-  // out of bounds, so the copy fills them with zeros without reading memory
+  if (ninputs < 1 || ninputs > kNI || (paired && ninputs % 2)) return cudaErrorInvalidValue;
+  // spec[freq][block][row][channel] float2 (paired: [row pair][channel][2]) as a
+  // 4-D FP32 tensor, innermost first: {2N floats (4N), ninputs rows (/ 2), nblk
+  // blocks, nfreqs}; box {a channel pair, 128 rows (64), kKT blocks, 1}: the rows
+  // beyond the job's inputs (and blocks beyond nblk) are out of bounds, so the
+  // copy fills them with zeros without reading memory
   CUtensorMap map;
-  const cuuint64_t dims[4] = {(cuuint64_t)(2 * N), (cuuint64_t)ninputs, (cuuint64_t)nblk, (cuuint64_t)nfreqs};
-  const int rp = tc_row_pairs();
-  const cuuint32_t box[4] = {(cuuint32_t)(4 * rp), (cuuint32_t)kNI, (cuuint32_t)kKT, 1};
-  {
-    cudaError_t e = tma_map_f32_4d(&map, spec, dims, box);
-    if (e != cudaSuccess) return e;
-  }
+  const int per = paired ? 2 : 1;
+  const cuuint64_t dims[4] = {(cuuint64_t)(2 * N * per), (cuuint64_t)(ninputs / per), (cuuint64_t)nblk, (cuuint64_t)nfreqs};
+  const cuuint32_t box[4] = {(cuuint32_t)(4 * per), (cuuint32_t)(kNI / per), (cuuint32_t)kKT, 1};
+  cudaError_t e = tma_map_f32_4d(&map, spec, dims, box);
+  if (e != cudaSuccess) return e;
   const size_t sm = xmac_tc_smem_bytes(hilo);
-  // converter warps: 8 unless GX_TC_CONV_WARPS=16 (measured no faster on C3)
-  const char *ce = getenv("GX_TC_CONV_WARPS");
-  const int cw = (ce && atoi(ce) == 16) ? 16 : 8;
-  dim3 grid(N / 2, nfreqs, ks);
-#define GX_TC_CASE(H, RPV, CWV)                                                                             \
-  if (hilo == H && rp == RPV && cw == CWV) {                                                                \
-    cudaError_t e = smem_opt_in((const void *)xmac_tc_kernel<H, RPV, CWV>, sm);                             \
-    if (e != cudaSuccess) return e;                                                                         \
-    xmac_tc_kernel<H, RPV, CWV><<<grid, tc_threads(CWV), sm, st>>>(map, nblk, N / 2, nfreqs, ks, ninputs,   \
-                                                                    scale, acc, accumulate, upper ? 1 : 0, err); \
-    return cudaGetLastError();                                                                              \
-  }
-  GX_TC_CASE(true, 1, 16) GX_TC_CASE(false, 1, 16) GX_TC_CASE(true, 1, 8) GX_TC_CASE(false, 1, 8)
-  GX_TC_CASE(true, 2, 16) GX_TC_CASE(false, 2, 16) GX_TC_CASE(true, 2, 8) GX_TC_CASE(false, 2, 8)
-#undef GX_TC_CASE
-  return cudaErrorInvalidValue;
+  auto go = [&](auto kernel) -> cudaError_t {
+    e = smem_opt_in((const void *)kernel, sm);
+    if (e != cudaSuccess) return e;
+    kernel<<<dim3(N / 2, nfreqs, ks), kTcThreads, sm, st>>>(map, nblk, N / 2, nfreqs, ks, ninputs, scale, acc, accumulate,
+                                                            upper ? 1 : 0, err);
+    return cudaGetLastError();
+  };
+  if (paired) return hilo ? go(xmac_tc_kernel<true, true>) : go(xmac_tc_kernel<false, true>);
+  return hilo ? go(xmac_tc_kernel<true, false>) : go(xmac_tc_kernel<false, false>);
 }
 
 cudaError_t finalise_tc_launch(const TcProdEntry *prods, const TcRowEntry *rows, int nrows, const float4 *acc,

@@ -312,9 +312,10 @@ __global__ void finalise_vis_kernel(const ProdEntry *__restrict__ prods, int npr
   float2 *out = results + pe.result_offset + c0;
   float2 s[4];
 #pragma unroll
-  for (int i = 0; i < 4; i++) s[i] = make_float2(0.f, 0.f);
-#pragma unroll 8
-  for (int k = 0; k < ks_count; k++) {
+  for (int i = 0; i < 4; i++)
+    s[i] = c0 + i * (int)blockDim.x < N ? a[i * blockDim.x] : make_float2(0.f, 0.f);
+#pragma unroll 2
+  for (int k = 1; k < ks_count; k++) {
 #pragma unroll
     for (int i = 0; i < 4; i++)
       if (c0 + i * (int)blockDim.x < N) {

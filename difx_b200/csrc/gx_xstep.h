@@ -76,13 +76,14 @@ struct TcRowEntry {
   int freq, a, bmin, start, end;
 };
 
-// Tensor-core X-step over spectra [freq][block][ninputs][N] (ninputs <= 128,
-// the MMA tile's M; missing rows are zeros); acc holds, per K-split slice,
+// Tensor-core X-step over spectra [freq][block][ninputs][N] (paired:
+// [freq][block][ninputs / 2][N][2]; ninputs <= 128, the MMA tile's M; missing
+// rows are zeros); acc holds, per K-split slice,
 // [freq][N/2][128][128] float4 = (Re, Im) of both channels of a channel pair,
 // unscaled, of which rows and columns below ninputs are written (upper: only
 // the 8 x 8 tiles on and above the diagonal).
 size_t xmac_tc_smem_bytes(bool hilo);
-cudaError_t xmac_tc_launch(const float2 *spec, int nblk, int N, int nfreqs, int ninputs, int ks, bool hilo,
+cudaError_t xmac_tc_launch(const float2 *spec, int nblk, int N, int nfreqs, int ninputs, bool paired, int ks, bool hilo,
                            const float *scale, float4 *acc, int accumulate, bool upper, int *err, cudaStream_t st);
 cudaError_t finalise_tc_launch(const TcProdEntry *prods, const TcRowEntry *rows, int nrows, const float4 *acc,
                                int nfreqs, int N, int ninputs, int ks, float2 *results, cudaStream_t st);
