@@ -40,11 +40,15 @@ constexpr int kMaxThreadId = 1023;
 
 enum SlotCode : int32_t { kGood = 0, kFillEnd = 1, kFillStart = 2, kForeign = 3, kInvalid = 4, kWrongThread = 5 };
 
+// The host copies all of these back, so they are small: 16 bytes a frame.
 struct SlotRecord {
-  int32_t code;
-  int32_t chan;
   int64_t frame;   // seconds x frames per second + frame number
+  uint32_t w3;     // header word 3
+  uint8_t code, chan;
+  uint8_t w1;      // header word 1, bits 24-31
+  uint8_t w02;     // header word 0 bit 30, then word 2 bits 29-31
 };
+static_assert(sizeof(SlotRecord) == 16, "one 16-byte store a frame");
 
 __global__ void vmux_classify_kernel(const uint8_t *__restrict__ src, long long nslots, int ifb, int fps, int nbits,
                                      int cpt, int enable_validity, const uint16_t *__restrict__ chan_of_thread,
@@ -54,9 +58,12 @@ __global__ void vmux_classify_kernel(const uint8_t *__restrict__ src, long long 
   if (k >= nslots) return;
   const uint8_t *f = src + k * (long long)ifb;
   const uint32_t *w = reinterpret_cast<const uint32_t *>(f);
-  SlotRecord r{kGood, -1, 0};
+  SlotRecord r{0, 0, kGood, 0xFF, 0, 0};
   const uint32_t last = *reinterpret_cast<const uint32_t *>(f + ifb - 4);
   const uint32_t w0 = w[0], w1 = w[1], w2 = w[2], w3 = w[3];
+  r.w3 = w3;
+  r.w1 = (uint8_t)(w1 >> 24);
+  r.w02 = (uint8_t)(((w0 >> 30) & 1u) | ((w2 >> 29) << 1));
   if (last == kFill) {
     r.code = kFillEnd;
   } else if (w0 == kFill) {
@@ -71,7 +78,7 @@ __global__ void vmux_classify_kernel(const uint8_t *__restrict__ src, long long 
     const int chan = chan_of_thread[tid];
     r.frame = (long long)(w0 & 0x3FFFFFFFu) * fps + (long long)(w1 & 0xFFFFFFu);
     if (chan == 0xFFFF) r.code = kWrongThread;
-    else r.chan = chan;
+    else r.chan = (uint8_t)chan;
   }
   rec[k] = r;
 }
@@ -121,18 +128,19 @@ __global__ void vmux_output_kernel(const uint8_t *__restrict__ src, uint8_t *__r
 // across the warp) and writes the P output words those 32 / B samples make;
 // every shift is a constant after unrolling, so the transpose stays in
 // registers.  Header words are written by the threads of q < 8.
-template <int P, int B>
+// Bound by HBM; VEC: the output frames are 16-byte aligned, and a thread's words
+// leave in 16-byte stores (as single words each store of a warp touched 32
+// sectors for 128 bytes).
+template <int P, int B, bool VEC>
 __global__ void __launch_bounds__(256) vmux_turn_kernel(const uint8_t *__restrict__ src, uint8_t *__restrict__ dest,
-                                                        int nout, int ofb, int ifb, int nthreads,
+                                                        int ofb, int ifb, int nthreads,
                                                         const int32_t *__restrict__ slot,
                                                         const uint32_t *__restrict__ hdr, int copy_missing_from_src)
 {
   constexpr int G = 32 / B;                       // samples per input word
   constexpr uint32_t M = B == 32 ? 0xFFFFFFFFu : ((1u << B) - 1u);
-  const int qwords = (ifb - kHeader) / 4;        // input payload words
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= (long long)nout * qwords) return;
-  const int f = (int)(t / qwords), q = (int)(t % qwords);
+  const int f = blockIdx.x, q = blockIdx.y * blockDim.x + threadIdx.x;
+  if (q >= (ifb - kHeader) / 4) return;          // input payload words
   uint32_t *out = reinterpret_cast<uint32_t *>(dest + (long long)f * ofb);
   const uint32_t h0 = hdr[(long long)f * 8];
   if (q < kHeader / 4) out[q] = hdr[(long long)f * 8 + q];
@@ -152,16 +160,25 @@ __global__ void __launch_bounds__(256) vmux_turn_kernel(const uint8_t *__restric
   }
   uint32_t *o = out + kHeader / 4 + (long long)q * P;
   // output group n = s * P + k (sample s of this word, thread k) sits at bits n * B
+  uint32_t v[P];
 #pragma unroll
   for (int j = 0; j < P; j++) {                 // output word j of this input word
-    uint32_t v = 0u;
+    v[j] = 0u;
 #pragma unroll
     for (int i = 0; i < G; i++) {
       const int n = j * G + i;
       const int s = n / P, k = n % P;
-      v |= ((in[k] >> (s * B)) & M) << (i * B);
+      v[j] |= ((in[k] >> (s * B)) & M) << (i * B);
     }
-    o[j] = v;
+  }
+  if constexpr (VEC && P >= 4) {
+#pragma unroll
+    for (int j = 0; j < P; j += 4) reinterpret_cast<uint4 *>(o)[j / 4] = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+  } else if constexpr (VEC && P == 2) {
+    *reinterpret_cast<uint2 *>(o) = make_uint2(v[0], v[1]);
+  } else {
+#pragma unroll
+    for (int j = 0; j < P; j++) o[j] = v[j];
   }
 }
 
@@ -173,10 +190,12 @@ struct gx_vdifmux {
   int ids[64] = {};
   int P = 1, B = 1, nout_chan = 1, ofb = 0, ids_bytes = 0, granularity = 1;
   uint16_t *d_chan = nullptr;
-  SlotRecord *d_rec = nullptr;
+  // pinned on the host: copies to and from pageable memory are staged by the
+  // driver and took longer than the kernels
+  SlotRecord *d_rec = nullptr, *h_rec = nullptr;
   long long rec_cap = 0;
-  int32_t *d_slot = nullptr;
-  uint32_t *d_hdr = nullptr;
+  // per output frame: the source slots of its threads, then its header (one copy)
+  uint32_t *d_out = nullptr, *h_out = nullptr;
   long long out_cap = 0;
   std::string err;
   gx_vdifmux_stats acc{};   // the accumulating counters
@@ -208,11 +227,12 @@ long long gcdll(long long a, long long b)
 
 // The reference's getLowestFrameNumber / getHighestFrameNumber over the slot
 // records: the extreme frame number among the first nSort usable frames.
-long long extreme_frame(const std::vector<SlotRecord> &rec, int nsort, bool highest)
+long long extreme_frame(const SlotRecord *rec, long long nrec, int nsort, bool highest)
 {
   long long best = -1;
   int n = 0;
-  for (const SlotRecord &r : rec) {
+  for (long long k = 0; k < nrec; k++) {
+    const SlotRecord &r = rec[k];
     if (r.code == kFillEnd || r.code == kFillStart || r.code == kForeign || r.code == kInvalid) continue;
     // frames of other threads count here: this scan does not look at threads
     const long long fn = r.frame;
@@ -297,23 +317,27 @@ gx_status gx_vdifmux_run(gx_vdifmux *m, const uint8_t *src, long long src_bytes,
   const int ifb = m->ifb;
   // ---- 1. classify every whole frame slot on the device
   const long long nslots = src_bytes >= ifb ? src_bytes / ifb : 0;
-  std::vector<SlotRecord> rec(nslots);
   if (nslots > 0) {
     if (nslots > m->rec_cap) {
       cudaFree(m->d_rec);
-      m->d_rec = nullptr;
+      cudaFreeHost(m->h_rec);
+      m->d_rec = m->h_rec = nullptr;
+      m->rec_cap = 0;
       if ((r = m->cuda(cudaMalloc(&m->d_rec, sizeof(SlotRecord) * nslots), "cudaMalloc")) != GX_OK) return r;
+      if ((r = m->cuda(cudaMallocHost(&m->h_rec, sizeof(SlotRecord) * nslots), "cudaMallocHost")) != GX_OK) return r;
       m->rec_cap = nslots;
     }
     const int tpb = 256;
     vmux_classify_kernel<<<(unsigned)((nslots + tpb - 1) / tpb), tpb, 0, st>>>(
         src, nslots, ifb, m->fps, m->nbits, m->cpt, (m->flags & GX_VDIFMUX_ENABLEVALIDITY) ? 1 : 0, m->d_chan, m->d_rec);
     if ((r = m->cuda(cudaGetLastError(), "vmux_classify_kernel")) != GX_OK) return r;
-    if ((r = m->cuda(cudaMemcpyAsync(rec.data(), m->d_rec, sizeof(SlotRecord) * nslots, cudaMemcpyDeviceToHost, st),
+    if ((r = m->cuda(cudaMemcpyAsync(m->h_rec, m->d_rec, sizeof(SlotRecord) * nslots, cudaMemcpyDeviceToHost, st),
                      "cudaMemcpyAsync")) != GX_OK)
       return r;
     if ((r = m->cuda(cudaStreamSynchronize(st), "cudaStreamSynchronize")) != GX_OK) return r;
   }
+
+  const SlotRecord *rec = m->h_rec;
 
   // ---- 2. the reference's sequential decisions over the records
   const int nthr = m->nthreads;
@@ -330,20 +354,32 @@ gx_status gx_vdifmux_run(gx_vdifmux *m, const uint8_t *src, long long src_bytes,
   const long long maxDest = dest_bytes / m->ofb - 1;
   long long startFrame = start_frame;
   if (startFrame < 0) {
-    startFrame = extreme_frame(rec, m->nsort, false);
+    startFrame = extreme_frame(rec, nslots, m->nsort, false);
     if (startFrame < 0) return m->fail(GX_ERR_IO, "no usable VDIF frame found");
   }
   const long long ntab = maxDest + 1 > 0 ? maxDest + 1 : 0;
   std::vector<uint64_t> mask(ntab, 0);
-  std::vector<int32_t> slot((size_t)ntab * nthr, -1);
+  if (ntab > m->out_cap) {
+    cudaFree(m->d_out);
+    cudaFreeHost(m->h_out);
+    m->d_out = m->h_out = nullptr;
+    m->out_cap = 0;
+    const size_t bytes = sizeof(uint32_t) * (size_t)ntab * (nthr + 8);
+    if ((r = m->cuda(cudaMalloc(&m->d_out, bytes), "cudaMalloc")) != GX_OK) return r;
+    if ((r = m->cuda(cudaMallocHost(&m->h_out, bytes), "cudaMallocHost")) != GX_OK) return r;
+    m->out_cap = ntab;
+  }
+  int32_t *slot = reinterpret_cast<int32_t *>(m->h_out);
+  std::fill(slot, slot + (size_t)ntab * nthr, -1);
   long long nValid = 0, nSkip = 0, nFill = 0, nDup = 0, nInvalid = 0, nDiscard = 0, nSeqUnproc = 0, nWrong = 0;
   long long highest = 0, bytesProcessed = -1, firstGoodByte = -1, nEnd = 0, highestSorted = -1;
   long long framesIn = 0;
   int protoSlot = -1;
   long long i = 0;
-  for (; i <= N;) {
-    const long long k = i / ifb;
-    const SlotRecord &rc = rec[k];
+  const SlotRecord *next = rec;
+  for (; i <= N;) {   // i stays a multiple of ifb
+    const SlotRecord &rc = *next++;
+    const long long k = &rc - rec;
     if (rc.code == kFillEnd || rc.code == kFillStart) { i += ifb; nFill += ifb; continue; }
     if (rc.code == kForeign) { i += ifb; nSkip += ifb; continue; }
     if (rc.code == kInvalid) { i += ifb; nInvalid++; continue; }
@@ -415,11 +451,15 @@ gx_status gx_vdifmux_run(gx_vdifmux *m, const uint8_t *src, long long src_bytes,
 
   // output headers: the prototype (first usable frame) with this mux's
   // channel count, thread 0, frame size and each frame's time and validity
+  // (of its words 0-2 only the bits in the record survive)
   uint32_t proto[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  if (protoSlot >= 0 &&
-      (r = m->cuda(cudaMemcpy(proto, src + (long long)protoSlot * ifb, 16, cudaMemcpyDeviceToHost), "cudaMemcpy")) !=
-          GX_OK)
-    return r;
+  if (protoSlot >= 0) {
+    const SlotRecord &pr = rec[protoSlot];
+    proto[0] = (uint32_t)(pr.w02 & 1u) << 30;
+    proto[1] = (uint32_t)pr.w1 << 24;
+    proto[2] = (uint32_t)(pr.w02 >> 1) << 29;
+    proto[3] = pr.w3;
+  }
   if (propagate) {   // EDV4 words: mask length (bits 16-23), extension version 4, sync word, validity mask
     proto[4] = (((uint32_t)nthr & 0xFFu) << 16) | (4u << 24);
     proto[5] = 0xACABFEEDu;
@@ -432,7 +472,7 @@ gx_status gx_vdifmux_run(gx_vdifmux *m, const uint8_t *src, long long src_bytes,
   proto[3] &= ~(1023u << 16);                                     // thread 0
   const int epoch = protoSlot >= 0 ? (int)((proto[1] >> 24) & 63u) : -1;
   const long long nout = highest + 1;
-  std::vector<uint32_t> hdr((size_t)std::max(0LL, nout) * 8);
+  uint32_t *hdr = m->h_out + (size_t)std::max(0LL, nout) * nthr;   // behind the slots in use
   long long nGood = 0, nPartial = 0, nBad = 0;
   long long secs = startFrame / m->fps, fnum = startFrame % m->fps;
   for (long long f = 0; f < nout; f++) {
@@ -466,33 +506,29 @@ gx_status gx_vdifmux_run(gx_vdifmux *m, const uint8_t *src, long long src_bytes,
 
   // ---- 3. headers and corner turn on the device
   if (nout > 0) {
-    if (nout > m->out_cap) {
-      cudaFree(m->d_slot);
-      cudaFree(m->d_hdr);
-      m->d_slot = nullptr;
-      m->d_hdr = nullptr;
-      if ((r = m->cuda(cudaMalloc(&m->d_slot, sizeof(int32_t) * nout * nthr), "cudaMalloc")) != GX_OK) return r;
-      if ((r = m->cuda(cudaMalloc(&m->d_hdr, sizeof(uint32_t) * 8 * nout), "cudaMalloc")) != GX_OK) return r;
-      m->out_cap = nout;
-    }
-    if ((r = m->cuda(cudaMemcpyAsync(m->d_slot, slot.data(), sizeof(int32_t) * nout * nthr, cudaMemcpyHostToDevice, st),
+    if ((r = m->cuda(cudaMemcpyAsync(m->d_out, m->h_out, sizeof(uint32_t) * (size_t)nout * (nthr + 8),
+                                     cudaMemcpyHostToDevice, st),
                      "cudaMemcpyAsync")) != GX_OK)
       return r;
-    if ((r = m->cuda(cudaMemcpyAsync(m->d_hdr, hdr.data(), sizeof(uint32_t) * 8 * nout, cudaMemcpyHostToDevice, st),
-                     "cudaMemcpyAsync")) != GX_OK)
-      return r;
+    const int32_t *d_slot = reinterpret_cast<const int32_t *>(m->d_out);
+    const uint32_t *d_hdr = m->d_out + (size_t)nout * nthr;
     const int tpb = 256;
-    const long long turns = nout * (long long)((ifb - kHeader) / 4);
-    const unsigned tgrid = (unsigned)((turns + tpb - 1) / tpb);
+    const dim3 tgrid((unsigned)nout, (unsigned)(((ifb - kHeader) / 4 + tpb - 1) / tpb));
+    const bool vec = ((uintptr_t)dest | (uintptr_t)m->ofb) % 16 == 0;
     bool done = false;
 #define GX_TURN(PP, BB)                                                                                     \
     if (!done && m->P == PP && m->B == BB) {                                                                \
-      vmux_turn_kernel<PP, BB><<<tgrid, tpb, 0, st>>>(src, dest, (int)nout, m->ofb, ifb, nthr, m->d_slot,   \
-                                                     m->d_hdr, propagate ? 1 : 0);                          \
+      if (vec)                                                                                              \
+        vmux_turn_kernel<PP, BB, true><<<tgrid, tpb, 0, st>>>(src, dest, m->ofb, ifb, nthr, d_slot, d_hdr,  \
+                                                              propagate ? 1 : 0);                           \
+      else                                                                                                  \
+        vmux_turn_kernel<PP, BB, false><<<tgrid, tpb, 0, st>>>(src, dest, m->ofb, ifb, nthr, d_slot, d_hdr, \
+                                                               propagate ? 1 : 0);                          \
       done = true;                                                                                          \
     }
     // every payload has at least 8 words, so the threads q < 8 cover the header
-    if ((ifb - kHeader) / 4 >= kHeader / 4) {
+    // (payloads of more than 64 MB are past the grid's limit)
+    if ((ifb - kHeader) / 4 >= kHeader / 4 && tgrid.y <= 65535) {
       GX_TURN(1, 1) GX_TURN(2, 1) GX_TURN(4, 1) GX_TURN(8, 1) GX_TURN(16, 1)
       GX_TURN(1, 2) GX_TURN(2, 2) GX_TURN(4, 2) GX_TURN(8, 2) GX_TURN(16, 2) GX_TURN(32, 2)
       GX_TURN(1, 4) GX_TURN(2, 4) GX_TURN(4, 4) GX_TURN(8, 4) GX_TURN(16, 4) GX_TURN(32, 4)
@@ -504,7 +540,7 @@ gx_status gx_vdifmux_run(gx_vdifmux *m, const uint8_t *src, long long src_bytes,
     if (!done) {   // other thread counts and sample widths: one thread per output word
       const long long words = nout * (long long)(m->ofb / 4);
       vmux_output_kernel<<<(unsigned)((words + tpb - 1) / tpb), tpb, 0, st>>>(src, dest, (int)nout, m->ofb, ifb, nthr,
-                                                                             m->P, m->B, m->d_slot, m->d_hdr,
+                                                                             m->P, m->B, d_slot, d_hdr,
                                                                              propagate ? 1 : 0);
     }
     if ((r = m->cuda(cudaGetLastError(), "vmux corner turn")) != GX_OK) return r;
@@ -533,7 +569,7 @@ gx_status gx_vdifmux_run(gx_vdifmux *m, const uint8_t *src, long long src_bytes,
   a.start_frame = startFrame;
   long long ret = bytesProcessed > firstGoodByte ? bytesProcessed : firstGoodByte;
   if (a.output_frames == 0 || bytesProcessed == 0 || firstGoodByte < 0 || nSeqUnproc >= nsort) {
-    const long long hi = extreme_frame(rec, m->nsort, true);
+    const long long hi = extreme_frame(rec, nslots, m->nsort, true);
     if (hi < 0) a.start_frame += (src_bytes / ifb) / nthr + 1;
     else a.start_frame = hi + 1;
     a.output_frames = 0;
@@ -561,8 +597,9 @@ gx_status gx_vdifmux_close(gx_vdifmux *m)
     cudaSetDevice(m->device);
     cudaFree(m->d_chan);
     cudaFree(m->d_rec);
-    cudaFree(m->d_slot);
-    cudaFree(m->d_hdr);
+    cudaFreeHost(m->h_rec);
+    cudaFree(m->d_out);
+    cudaFreeHost(m->h_out);
   }
   delete m;
   return GX_OK;
