@@ -273,6 +273,8 @@ static gx_status setup(gx_handle *h)
   int ni = 0;
   for (int f = 0; f < d.nfreqs; f++) ni = count[f] > ni ? count[f] : ni;
   J.nrows = ni;
+  bool rows_full = true;   // every freq uses the same rows: each pass writes all that the X-steps read
+  for (int f = 0; f < h->nfmain; f++) rows_full = rows_full && count[f] == ni;
   if (d.xstep < GX_XSTEP_FP32 || d.xstep > GX_XSTEP_AUTO) return h->fail(GX_ERR_ARG, "unknown xstep");
   h->xstep = d.xstep;
   if (d.xstep == GX_XSTEP_AUTO) {
@@ -1102,7 +1104,7 @@ static gx_status setup(gx_handle *h)
   }
   const size_t spec_elems = (size_t)h->nfmain * chunk * J.ninputs * J.nchan;
   CKR(h, h->dalloc(&h->d_spec, sizeof(float2) * spec_elems));
-  CKR(h, cudaMemsetAsync(h->d_spec, 0, sizeof(float2) * spec_elems, h->stream));
+  if (!rows_full) CKR(h, cudaMemsetAsync(h->d_spec, 0, sizeof(float2) * spec_elems, h->stream));
   CKR(h, h->dalloc(&h->d_spec1, sizeof(float2) * (size_t)h->nfmain * J.ninputs * J.nchan));
   CKR(h, cudaMemsetAsync(h->d_spec1, 0, sizeof(float2) * (size_t)h->nfmain * J.ninputs * J.nchan, h->stream));
   CKR(h, h->dalloc(&h->d_w, sizeof(float) * (size_t)h->nwrows * chunk));
