@@ -12,13 +12,14 @@
 // registers a thread leave 16 warps an SM, so what is left is latency (issue
 // active 45-60 %, FMA pipe 42-54 %).  F-step times against the kernels it
 // replaced, which took one band at a time and built the rotator tables of
-// transforms below 512 points once per band (1 B200):
-//   4 stations, 2-bit, 256 points, 200 ms subint     2.77 -> 0.59 ms
-//   11 stations, 1-bit, 128 points, 200 ms           5.00 -> 0.97 ms
-//   16 stations, 2-bit, 512 points, 50 ms            2.13 -> 1.61 ms
-//   6 stations, INTERLACEDVDIF, 1024 points, 100 ms  1.64 -> 0.83 ms
-//   64 stations, 8-bit complex, 4096 points, 32 ms   4.03 -> 3.54 ms
-//   64 stations, 2-bit, 8192 points, 32 ms           7.25 -> 7.10 ms
+// transforms below 512 points once per band (1 B200; the short transforms'
+// now in passes of up to 32768 blocks, in passes of 4096 as before in brackets):
+//   4 stations, 2-bit, 256 points, 200 ms subint     2.77 -> 0.37 ms (0.59)
+//   11 stations, 1-bit, 128 points, 200 ms           5.00 -> 0.73 ms (0.97)
+//   16 stations, 2-bit, 512 points, 50 ms            2.13 -> 1.55 ms (1.61)
+//   6 stations, INTERLACEDVDIF, 1024 points, 100 ms  1.64 -> 0.75 ms (0.83)
+//   64 stations, 8-bit complex, 4096 points, 32 ms   4.03 -> 3.57 ms
+//   64 stations, 2-bit, 8192 points, 32 ms           7.25 -> 7.13 ms
 //
 // Per pair of bands a group
 //   1. decodes its field of 16 time samples held in registers (one 32-bit

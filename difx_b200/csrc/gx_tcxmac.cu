@@ -184,7 +184,7 @@ constexpr int kNumBars = 2 * kRingStages + 2 * kOpStages + 1;   // full, empty, 
 // paired-band F-step writes the two polarisations of a station.  A tile is then
 // 1024 rows of 32 bytes instead of 2048 of 16: the tile loads bound the kernel, at
 // a rate of rows, and 16-byte rows move half-used sectors (64 stations, 4096
-// channels, 500 blocks: X stage 3.01 -> 2.58 ms split, 2.66 -> 1.93 ms single).
+// channels, 500 blocks: X stage 3.01 -> 2.47 ms split, 2.66 -> 1.93 ms single).
 template <bool HILO, bool PAIRED>
 __global__ void __launch_bounds__(kTcThreads, 1)
 xmac_tc_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int NP, int nfreqs, int ks, int ninputs,
