@@ -30,7 +30,7 @@ REFERENCE_SRC = os.environ.get("DIFX_REFERENCE", "/root/reference")
 def build(reference: bool = True) -> None:
     """Build the oracle (and, where the reference tree exists, the reference harness)."""
     subprocess.run(["make", "-s", "-C", HERE], check=True)
-    if reference and os.path.isdir(REFERENCE_SRC):
+    if reference and os.path.isdir(os.path.join(REFERENCE_SRC, "mpifxcorr")):
         subprocess.run(["make", "-s", "-C", HERE, "ref", "-j8", f"REF={REFERENCE_SRC}"], check=True)
         subprocess.run(["make", "-s", "-C", HERE, "vmux", f"REF={REFERENCE_SRC}"], check=True)
         subprocess.run(["make", "-s", "-C", HERE, "shim", "-j8", f"REF={REFERENCE_SRC}"], check=True)
