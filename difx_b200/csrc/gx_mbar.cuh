@@ -6,6 +6,7 @@
 #include <cstdint>
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include "gx_warp_wait.h"
 
 namespace gx {
 namespace {
@@ -55,6 +56,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity)
   while (!mbar_try_wait(bar, parity))
     if (global_ns() - t0 > kWaitLimitNs) return false;
   return true;
+}
+
+// The same for a whole warp, with one answer for all its lanes: false too once
+// the CTA's abort flag is set.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, const volatile int *abort)
+{
+  return warp_agrees([&] { return mbar_wait(bar, parity); }, [&] { return *abort != 0; },
+                     [](bool good) { return __all_sync(0xffffffffu, good) != 0; });
 }
 
 // One tile of a 4-D tensor map (no multicast) into shared memory; coordinates innermost first.

@@ -180,7 +180,7 @@ xmac_fp32_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int N, 
 #pragma unroll 1
     for (; st < run; st++) {
       const int buf = st % NSTAGE;
-      if (!mbar_wait(smem_u32(full + buf), (uint32_t)(st / NSTAGE) & 1u) || *s_abort) {
+      if (!mbar_wait_warp(smem_u32(full + buf), (uint32_t)(st / NSTAGE) & 1u, s_abort)) {
         abort_with(14);
         ok = false;
         break;
