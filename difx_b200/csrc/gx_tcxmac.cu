@@ -233,7 +233,7 @@ xmac_tc_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int NP, i
   const uint32_t tmem = *s_tmem;
   auto abort_with = [&](int code) {
     *s_abort = 1;
-    atomicExch(err, code);
+    atomicCAS(err, 0, code);   // the first status stays
   };
 
   int issued = 0, mmas = 0;
@@ -301,9 +301,8 @@ xmac_tc_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int NP, i
     };
     const uint32_t at0 = place(r, e0), at1 = place(r1, e1);
     for (int t = 0; t < nt; t++) {
-      if (*s_abort) break;
       const int st = t % kStages, o = t % kOpStages;
-      if (!mbar_wait(smem_u32(full + st), (uint32_t)(t / kStages) & 1u)) {
+      if (!mbar_wait_warp(smem_u32(full + st), (uint32_t)(t / kStages) & 1u, s_abort)) {
         abort_with(1);
         break;
       }
@@ -334,7 +333,7 @@ xmac_tc_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int NP, i
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(empty + st));   // the staging stage may be reloaded
-      if (t >= kOpStages && !mbar_wait(smem_u32(opempty + o), (uint32_t)(t / kOpStages - 1) & 1u)) {
+      if (t >= kOpStages && !mbar_wait_warp(smem_u32(opempty + o), (uint32_t)(t / kOpStages - 1) & 1u, s_abort)) {
         abort_with(2);
         break;
       }
@@ -362,7 +361,8 @@ xmac_tc_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int NP, i
   }
   __syncthreads();
   // all MMAs of the slice have completed once the last commit has arrived
-  if (!*s_abort && nt > 0 && tid == 0 && !mbar_wait(smem_u32(done), 0u)) abort_with(5);
+  if (tid == 0 && nt > 0 && !*s_abort && !mbar_wait(smem_u32(done), 0u)) abort_with(5);
+  __syncthreads();   // every thread sees whether that wait ran out
   if (*s_abort) {
     // drain: the loads this CTA issued, then the MMAs it committed (bounded)
     if (warp == 0 && lane == 0)

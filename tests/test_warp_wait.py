@@ -22,7 +22,7 @@ def test_lanes_leave_together(tmp_path):
     assert alone == patterns   # what the vote is there for
 
 
-@pytest.mark.parametrize("source,kernel", [("gx_xstep.cu", "xmac_fp32_kernel")])
+@pytest.mark.parametrize("source,kernel", [("gx_xstep.cu", "xmac_fp32_kernel"), ("gx_tcxmac.cu", "xmac_tc_kernel")])
 def test_whole_warps_wait_by_vote(source, kernel):
     """A wait before the kernel's full-mask warp barriers is the voting one."""
     src = open(os.path.join(ROOT, "difx_b200", "csrc", source)).read()
