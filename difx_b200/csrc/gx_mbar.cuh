@@ -58,12 +58,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity)
   return true;
 }
 
-// The same for a whole warp, with one answer for all its lanes: false too once
-// the CTA's abort flag is set.
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, const volatile int *abort)
+// Ends a stage for a whole warp: its barrier, and whether every lane goes on.
+__device__ __forceinline__ bool stage_end(bool good)
 {
-  return warp_agrees([&] { return mbar_wait(bar, parity); }, [&] { return *abort != 0; },
-                     [](bool good) { return __all_sync(0xffffffffu, good) != 0; });
+  return warp_goes_on(good, [](bool g) { return __all_sync(0xffffffffu, g) != 0; }, [] { __syncwarp(); });
 }
 
 // One tile of a 4-D tensor map (no multicast) into shared memory; coordinates innermost first.

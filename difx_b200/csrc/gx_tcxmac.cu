@@ -302,10 +302,7 @@ xmac_tc_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int NP, i
     const uint32_t at0 = place(r, e0), at1 = place(r1, e1);
     for (int t = 0; t < nt; t++) {
       const int st = t % kStages, o = t % kOpStages;
-      if (!mbar_wait_warp(smem_u32(full + st), (uint32_t)(t / kStages) & 1u, s_abort)) {
-        abort_with(1);
-        break;
-      }
+      const bool loaded = mbar_wait(smem_u32(full + st), (uint32_t)(t / kStages) & 1u) && !*s_abort;
       const int kv = min(kKT, nblk - (t0 + t) * kKT);
       const float4 *stg = reinterpret_cast<const float4 *>(staging + st * kStageBytes);
       // (value 0 re, im, value 1 re, im) at block k; of an odd piece of a pair, input r is the second
@@ -331,12 +328,12 @@ xmac_tc_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int NP, i
           im1[j] = pack_half2(a.w * s1, b.w * s1);
         }
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(empty + st));   // the staging stage may be reloaded
-      if (t >= kOpStages && !mbar_wait_warp(smem_u32(opempty + o), (uint32_t)(t / kOpStages - 1) & 1u, s_abort)) {
-        abort_with(2);
+      if (!stage_end(loaded)) {
+        abort_with(1);
         break;
       }
+      if (lane == 0) mbar_arrive(smem_u32(empty + st));   // the staging stage may be reloaded
+      const bool free = t < kOpStages || mbar_wait(smem_u32(opempty + o), (uint32_t)(t / kOpStages - 1) & 1u);
       unsigned char *op = ops + o * kOpStageBytes;
       // channel e, part q at op + (q * 2 + e) * kOpChanBytes; Xi rows 0..127, Xr rows 128..255
       auto put = [&](unsigned char *dst, const uint32_t (&w)[NW]) {
@@ -355,7 +352,10 @@ xmac_tc_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int NP, i
         put(lo + at1 + kXrOffset, lre1);
       }
       fence_proxy_async_smem();
-      __syncwarp();
+      if (!stage_end(free)) {
+        abort_with(2);
+        break;
+      }
       if (lane == 0) mbar_arrive(smem_u32(opfull + o));   // the operand stage may be multiplied
     }
   }

@@ -1,8 +1,12 @@
-// A wait that ends the same way for every lane of a warp.  A bounded wait can
+// A stage that ends the same way for every lane of a warp.  A bounded wait can
 // succeed in one lane and run out in its neighbour, and a lane can read the
 // abort flag a moment before or after it is set; lanes that decided alone would
 // then part -- some at the warp's next barrier, some at the CTA's -- and wait
-// for one another without limit.  So the lanes vote: all go on, or all leave.
+// for one another without limit.  So a lane whose wait ran out still works
+// through the stage (its sums are thrown away) and the lanes vote at the
+// barrier that ends it: all go on, or all leave.  (A vote in front of the work
+// instead put its latency on the stage's critical path: tensor-core X-step of 64
+// stations, 4096 channels, 250 blocks, 1.45 -> 1.48 ms.)
 #pragma once
 
 #ifdef __CUDACC__
@@ -13,14 +17,14 @@
 
 namespace gx {
 
-// wait: this lane's bounded wait (true: it succeeded); aborted: this lane's view
-// of the abort flag, read after the wait; all: true in every lane if every
-// lane's argument is.
-template <class Wait, class Aborted, class All>
-GX_HOST_DEVICE bool warp_agrees(Wait wait, Aborted aborted, All all)
+// good: this lane's wait succeeded and it saw no abort; all: true in every lane
+// if every lane's argument is; sync: the warp's barrier.
+template <class All, class Sync>
+GX_HOST_DEVICE bool warp_goes_on(bool good, All all, Sync sync)
 {
-  const bool good = wait() && !aborted();
-  return all(good);
+  const bool go = all(good);
+  sync();
+  return go;
 }
 
 }  // namespace gx

@@ -180,11 +180,7 @@ xmac_fp32_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int N, 
 #pragma unroll 1
     for (; st < run; st++) {
       const int buf = st % NSTAGE;
-      if (!mbar_wait_warp(smem_u32(full + buf), (uint32_t)(st / NSTAGE) & 1u, s_abort)) {
-        abort_with(14);
-        ok = false;
-        break;
-      }
+      const bool good = mbar_wait(smem_u32(full + buf), (uint32_t)(st / NSTAGE) & 1u) && !*s_abort;
       const float2 *bi_ = sI + buf * STAGE + ti * kTA * CT + c;
       const float2 *bj_ = sJ + buf * STAGE + tj * TB * CT + c;
 #pragma unroll 1
@@ -209,7 +205,11 @@ xmac_fp32_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int N, 
           for (int b = 0; b < TB; b++) acc2[a][b] = __ffma2_rn(xs, by[b], acc2[a][b]);
         }
       }
-      __syncwarp();
+      if (!stage_end(good)) {
+        abort_with(14);
+        ok = false;
+        break;
+      }
       if (lane == 0) {
         // done with the stage: the last warp to be (its acquire follows every
         // other's release, so all reads of the stage precede the copy) refills it

@@ -1,7 +1,6 @@
 // Host model of a consumer warp of the X-steps' stage rings: 32 threads stand
 // for its lanes, each with a bounded wait of its own that succeeds or runs out
-// per stage.  Lanes that go on meet at the warp's barrier, lanes that leave at
-// the CTA's.  Prints, for the vote of gx_warp_wait.h and for lanes that decide
+// per stage.  A stage ends at the warp's barrier, the loop at the CTA's.  Prints, for the vote of gx_warp_wait.h and for lanes that decide
 // alone, how many patterns of waits left a lane at a barrier for good.
 #include <chrono>
 #include <condition_variable>
@@ -47,14 +46,19 @@ static bool run(const std::vector<std::vector<bool>> &wait_ok, const std::vector
   for (int lane = 0; lane < kLanes; lane++)
     t.emplace_back([&, lane] {
       for (int st = 0; st < kStages; st++) {
-        const bool go = gx::warp_agrees([&] { return (bool)wait_ok[lane][st]; }, [&] { return (bool)abort_seen[lane][st]; },
-                                        [&](bool good) {
-                                          if (!vote) return good;
-                                          bool agreed = false;
-                                          return ballot.arrive(good, &agreed) && agreed;
-                                        });
+        const bool good = wait_ok[lane][st] && !abort_seen[lane][st];
+        bool met = true;
+        const bool go = gx::warp_goes_on(
+            good,
+            [&](bool g) {
+              if (!vote) return g;
+              bool agreed = false;
+              met = ballot.arrive(g, &agreed);
+              return met && agreed;
+            },
+            [&] { met = warp.arrive(true, nullptr) && met; });
+        if (!met) return;
         if (!go) break;
-        if (!warp.arrive(true, nullptr)) return;
       }
       done[lane] = cta.arrive(true, nullptr);
     });
@@ -70,7 +74,7 @@ int main()
   std::srand(3);
   for (int k = 0; k < 6; k++) {
     std::vector<std::vector<bool>> ok(kLanes, std::vector<bool>(kStages, true)), ab(kLanes, std::vector<bool>(kStages, false));
-    const int st = std::rand() % kStages;
+    const int st = std::rand() % (kStages - 1);
     for (int lane = 0; lane < kLanes; lane++) {
       if (k % 2 == 0) ok[lane][st] = std::rand() % 3 != 0;        // some lanes' waits run out
       else ab[lane][st] = std::rand() % 3 == 0;                   // some lanes see the flag earlier

@@ -23,12 +23,10 @@ def test_lanes_leave_together(tmp_path):
 
 
 @pytest.mark.parametrize("source,kernel", [("gx_xstep.cu", "xmac_fp32_kernel"), ("gx_tcxmac.cu", "xmac_tc_kernel")])
-def test_whole_warps_wait_by_vote(source, kernel):
-    """A wait before the kernel's full-mask warp barriers is the voting one."""
+def test_stages_end_by_vote(source, kernel):
+    """In the kernels whose warps wait per lane, no bare full-mask barrier ends a stage."""
     src = open(os.path.join(ROOT, "difx_b200", "csrc", source)).read()
     body = src[src.index(kernel + "("):]
     body = re.sub(r"//[^\n]*", "", body[:body.index("\n}\n")])
-    waits = [m.start() for m in re.finditer(r"mbar_wait\(", body)]
-    for b in (m.start() for m in re.finditer(r"__syncwarp\(\)", body)):
-        loop = body.rindex("for (", 0, body.rindex("mbar_wait", 0, b))
-        assert not [w for w in waits if loop < w < b], "a lane-by-lane wait before a warp barrier"
+    assert "mbar_wait(" in body and "stage_end(" in body
+    assert "__syncwarp" not in body
