@@ -19,7 +19,8 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libgxcorr.so")
 BUILD = os.path.join(HERE, "_build")
 
-SOURCES = ["gx_fstep.cu", "gx_fstep_pair.cu", "gx_fstep_pair_real.cu", "gx_fstep_pair_cplx.cu", "gx_fstep_pair_real_pc.cu", "gx_fstep_pair_cplx_pc.cu", "gx_xstep.cu", "gx_tcxmac.cu", "gx_noalloc.cu", "gx_vis.cu", "gx_api.cpp", "gx_input.cpp",
+SOURCES = ["gx_fstep.cu", "gx_fstep_pair.cu", "gx_fstep_pair_real.cu", "gx_fstep_pair_cplx.cu", "gx_fstep_pair_real_pc.cu", "gx_fstep_pair_cplx_pc.cu", "gx_fstep_pair_one.cu",
+           "gx_fstep_pair_one_pc.cu", "gx_xstep.cu", "gx_tcxmac.cu", "gx_noalloc.cu", "gx_vis.cu", "gx_api.cpp", "gx_input.cpp",
            "gx_server.cpp", "gx_batch.cpp", "gx_vdifmux.cu", "gx_ring.cu", "gx_monitor.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 

@@ -1,6 +1,7 @@
 // F-step of two bands at a time: one group of F / 16 threads per (station, FFT
 // block) transforms the station's bands in pairs (2p, 2p + 1), each thread
-// holding 16 points of both bands as packed FP32 pairs.
+// holding 16 points of both bands as packed FP32 pairs.  With an odd number of
+// bands the two lanes are two consecutive blocks of one band instead.
 //
 // What bounds it.  A 4096-point transform is about 60 FP32 operations and 16
 // bytes of shared-memory exchange a sample against 10 bytes of HBM, so the SM's
@@ -20,6 +21,18 @@
 //   6 stations, INTERLACEDVDIF, 1024 points, 100 ms  1.64 -> 0.75 ms (0.83)
 //   64 stations, 8-bit complex, 4096 points, 32 ms   4.03 -> 3.57 ms
 //   64 stations, 2-bit, 8192 points, 32 ms           7.25 -> 7.13 ms
+//
+// An odd band count as pairs, the last band alone in both lanes, transformed that
+// band twice and read its samples byte by byte between the decodes; as two
+// blocks of a band, with all of a thread's words on their way before the first
+// is used, against that and against one band at a time (16 stations, 8 bits,
+// F-step times):
+//   1 band, real, 2048 points, 4000 blocks     1.44 -> 0.52 ms (one at a time 0.60)
+//   1 band, real, 8192 points, 1000 blocks     1.80 -> 0.66 ms (0.60)
+//   1 band, complex, 1024 points, 8000 blocks  1.68 -> 0.55 ms (0.73)
+//   1 band, complex, 4096 points, 2000 blocks  1.71 -> 0.57 ms (0.72)
+//   3 bands, real, 1024 points, 4000 blocks    1.48 -> 0.70 ms (1.07)
+//   3 bands, complex, 1024 points, 2000 blocks 1.02 -> 0.43 ms (0.55)
 //
 // Per pair of bands a group
 //   1. decodes its field of 16 time samples held in registers (one 32-bit
@@ -53,19 +66,24 @@ cudaError_t smem_opt_in(const void *kernel, size_t bytes);
 
 // How a pair's field is found and decoded; the same for every station of a job.
 struct PairDecode {
-  int npairs;        // band pairs (the last one holds a single band when nbands is odd)
-  int width;         // bits of a pair's field
+  int nfields;       // band pairs, or bands where the lanes are two blocks of a band
+  int width;         // bits of a pair's or band's field
   int ts_bits;       // bits of a time sample
   int ncol, ppc;     // columns loaded per time sample, pairs per column
-  int load;          // alignment of the columns (1, 2 or 4 bytes), 0: bytes of the field one by one
+  int load;          // 1: pairs are read as aligned columns, 0: bytes of the field one by one
   int kind;          // 0: level pair from a table of 1- or 2-bit real codes, 1: 8-bit codes, 2: level table
   float scale;       // kind 1: level = (code - 128) scale, the scale carried by the rotator
 };
 
 namespace pr {
 
+// What the two lanes of a thread's packed values are.
+constexpr int kSameBands = 0;   // two bands of one frequency: one set of rotator tables
+constexpr int kTwoBands = 1;    // two bands, a set of tables each
+constexpr int kTwoBlocks = 2;   // two consecutive FFT blocks of one band, a set of tables each: odd band counts
+
 struct V {
-  float2 re, im;     // lanes: the two bands
+  float2 re, im;     // the two lanes
 };
 
 __device__ __forceinline__ float2 dup(float a) { return make_float2(a, a); }
@@ -253,12 +271,18 @@ struct Cfg {
   static_assert(NTS % S == 0, "");
 };
 
-template <int F, int CPLX>
-__host__ __device__ constexpr size_t smem_bytes(int sets)
+template <int F, int CPLX, int LANES>
+__host__ __device__ constexpr size_t group_bytes()
 {
   using C = Cfg<F, CPLX>;
-  return sizeof(float2) * (2 * kTwRow + C::FIN) +
-         (size_t)C::G * (C::XB * sizeof(float4) + (size_t)(C::TBUF * sets * C::T) * sizeof(float2) + 2 * sizeof(BlockParam));
+  return C::XB * sizeof(float4) + (size_t)(C::TBUF * (LANES == kSameBands ? 1 : 2) * C::T) * sizeof(float2) +
+         2 * (LANES == kTwoBlocks ? 2 : 1) * sizeof(BlockParam);
+}
+template <int F, int CPLX, int LANES>
+__host__ __device__ constexpr size_t smem_bytes()
+{
+  using C = Cfg<F, CPLX>;
+  return sizeof(float2) * (2 * kTwRow + C::FIN) + (size_t)C::G * group_bytes<F, CPLX, LANES>();
 }
 
 // Radix-16 pass of stride 16 (P = 1) or 256 (P = 2): twiddles from the rows
@@ -325,6 +349,16 @@ __device__ __forceinline__ void cp_async16(void *sdst, const void *gsrc)
 __device__ __forceinline__ void cp_async_wait_all()
 {
   asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+}
+
+// The word at p, or 0 without reading it.
+__device__ __forceinline__ uint32_t load_if(const void *p, bool pred)
+{
+  uint32_t v;
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\tmov.u32 %0, 0;\n\t@p ld.global.nc.u32 %0, [%1];\n\t}"
+               : "=r"(v)
+               : "l"(p), "r"((unsigned int)pred));
+  return v;
 }
 
 template <int NT, int CTA>
@@ -415,7 +449,7 @@ __device__ __forceinline__ int pc_slot(int m)
   return C::SPLIT ? (m & 1) * (C::FS + C::FS / 16) + 17 * (m >> 1) + 16 : 17 * m + 16;
 }
 
-template <int F, int CPLX, bool SAME, bool PC>
+template <int F, int CPLX, int LANES, bool PC>
 __global__ void __launch_bounds__(Cfg<F, CPLX>::CTA, Cfg<F, CPLX>::MINB)
 fstep_pair_kernel(const __grid_constant__ DevJob J, const DevStation *__restrict__ stations, SubintArrays S,
                   const BlockParam *__restrict__ bp, int nblk, int blocks_per_group, PairDecode D,
@@ -423,7 +457,9 @@ fstep_pair_kernel(const __grid_constant__ DevJob J, const DevStation *__restrict
 {
   using C = Cfg<F, CPLX>;
   constexpr int NT = C::NT, CTA = C::CTA, G = C::G, N = C::N, SD = C::S, LGS = C::LGS, T = C::T;
+  constexpr bool SAME = LANES == kSameBands;
   constexpr int SETS = SAME ? 1 : 2;
+  constexpr int NB = LANES == kTwoBlocks ? 2 : 1;   // blocks of a unit of a group's work
   constexpr bool HALF = !CPLX;
   constexpr int NOUT = CPLX ? 16 : 8;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -440,11 +476,10 @@ fstep_pair_kernel(const __grid_constant__ DevJob J, const DevStation *__restrict
   float2 *twA = reinterpret_cast<float2 *>(smem_raw);
   float2 *twB = twA + kTwRow;
   float2 *fin = twB + kTwRow;
-  constexpr size_t kGroup = C::XB * sizeof(float4) + (size_t)(C::TBUF * SETS * T) * sizeof(float2) + 2 * sizeof(BlockParam);
-  unsigned char *mine = reinterpret_cast<unsigned char *>(fin + C::FIN) + (size_t)g * kGroup;
+  unsigned char *mine = reinterpret_cast<unsigned char *>(fin + C::FIN) + (size_t)g * group_bytes<F, CPLX, LANES>();
   float4 *xb = reinterpret_cast<float4 *>(mine);
   float2 *tabs = reinterpret_cast<float2 *>(mine + C::XB * sizeof(float4));
-  // parameters of the group's current block and of its next one
+  // parameters of the group's current unit of NB blocks and of its next one
   BlockParam *const pbuf = reinterpret_cast<BlockParam *>(tabs + C::TBUF * SETS * T);
 
   for (int i = tid; i < 256; i += CTA) s_lut[i] = J.lut[i];
@@ -465,6 +500,7 @@ fstep_pair_kernel(const __grid_constant__ DevJob J, const DevStation *__restrict
 
   const uint8_t *data = S.data[s];
   const int fsamp = J.framesamples, fbytes = J.framebytes;
+  const int nunit = (nblk + NB - 1) / NB;
   // phase-cal: as the binning kernels form it
   const int pcfirst = PC ? pf.first[s] : -1;
   const int pcn = PC ? pf.nbins : 1;
@@ -487,18 +523,21 @@ fstep_pair_kernel(const __grid_constant__ DevJob J, const DevStation *__restrict
   uint32_t raw[16];        // words with the time samples' current column
   int rsh = 0;             // bits below the column (the same for all of a thread's samples)
   unsigned int vmask = 0;  // bit t: sample j + NT t is valid (before any per-band mask)
-  bool live = false;       // the block in raw is processed
-  const bool fast = D.load && NT <= fsamp;
-  // Copies block bi's parameters into a buffer (completes before the copying
+  unsigned int vmask1 = 0; // the same of a unit's second block
+  bool live = false;       // a block of the unit in raw (and the masks) is processed
+  const bool fast = NB == 1 && D.load && NT <= fsamp;
+  // Copies unit u's parameters into a buffer (completes before the copying
   // threads' cp_async_wait_all; state 0 where there is no such block).
-  auto fetch_param = [&](int bi, BlockParam *dst) {
-    if (j >= (int)(sizeof(BlockParam) / 16)) return;
-    if (bi < nblk) cp_async16(reinterpret_cast<char *>(dst) + 16 * j, reinterpret_cast<const char *>(bp + (size_t)s * nblk + bi) + 16 * j);
-    else reinterpret_cast<uint4 *>(dst)[j] = make_uint4(0u, 0u, 0u, 0u);
+  auto fetch_param = [&](int u, BlockParam *dst) {
+    constexpr int kPieces = (int)(sizeof(BlockParam) / 16);
+    for (int i = j; i < NB * kPieces; i += NT) {
+      if (u * NB + i / kPieces < nblk) cp_async16(reinterpret_cast<char *>(dst) + 16 * i, reinterpret_cast<const char *>(bp + (size_t)s * nblk + u * NB) + 16 * i);
+      else reinterpret_cast<uint4 *>(dst)[i] = make_uint4(0u, 0u, 0u, 0u);
+    }
   };
   // Loads column col of the samples j + NT t of the block P; samples of invalid
   // frames (and blocks that are not processed) are not read.
-  auto load_raw = [&](const BlockParam &P, int col) {
+  auto load_column = [&](const BlockParam &P, int col) {
     vmask = 0;
     live = P.state != 0;
     if (!live) return;
@@ -546,27 +585,80 @@ fstep_pair_kernel(const __grid_constant__ DevJob J, const DevStation *__restrict
       }
     }
   };
-  // Builds the rotator tables of pair p of the block P into buf.
-  auto build_tables = [&](const BlockParam &P, int p, float2 *buf) {
+  // Which of the thread's samples of the block P are valid.
+  auto valid_samples = [&](const BlockParam &P) {
+    const int nfr = P.nframes, smp0 = P.nearestsample + jb;
+    const unsigned long long vm = P.validmask;
+    if (P.state == 0) return 0u;
+    if (nfr >= 64 ? vm == ~0ull : vm == ((1ull << nfr) - 1ull)) return 0xFFFFu;
+    int q = smp0 / fsamp, r = smp0 - q * fsamp;
+    unsigned int m = 0;
+    q -= P.fr0;
+#pragma unroll 1
+    for (int t = 0; t < 16; t++) {
+      m |= (unsigned int)((vm >> min(q, 63)) & 1ull) << t;
+      r += NT;
+      while (r >= fsamp) {
+        r -= fsamp;
+        q++;
+      }
+    }
+    return m;
+  };
+  // Takes over the unit P: of one block, column col too; of two, their masks alone.
+  auto load_raw = [&](const BlockParam *P, int col) {
+    if constexpr (NB == 2) {
+      vmask = valid_samples(P[0]);
+      vmask1 = valid_samples(P[1]);
+      live = P[0].state != 0 || P[1].state != 0;
+    } else {
+      load_column(P[0], col);
+    }
+  };
+  // The words of a thread's 16 samples of the block P that hold the field at bit
+  // `off` of each time sample, in w, all on their way before the first is used; of
+  // samples not in vm 0.  A field starts at a multiple of its bits, a power of
+  // two, so it lies in one word.  Frames and their payloads are whole words, so a
+  // word ends within the frame and sample t's field starts at bit (start + NT t
+  // ts_bits) mod 32 in whichever frame it lies.  Returns that start.
+  auto load_words = [&](const BlockParam &P, int off, unsigned int vm, uint32_t (&w)[16]) {
+    const int smp0 = P.nearestsample + jb;
+    int q = smp0 / fsamp, r = smp0 - q * fsamp;
+    const uint8_t *fr = data + (long long)q * fbytes + 32;
+    const int start = (r * D.ts_bits + off) & 31;
+#pragma unroll
+    for (int t = 0; t < 16; t++) {
+      w[t] = load_if(fr + 4 * ((r * D.ts_bits + off) >> 5), (vm >> t) & 1u);
+      r += NT;
+#pragma unroll 1
+      while (r >= fsamp) {
+        r -= fsamp;
+        fr += fbytes;
+      }
+    }
+    return start;
+  };
+  // Builds the rotator tables of pair p of the unit P into buf.
+  auto build_tables = [&](const BlockParam *P, int p, float2 *buf) {
 #pragma unroll
     for (int k = 0; k < SETS; k++) {
-      const int bd = min(2 * p + k, J.nbands - 1);
-      put_entries<C>(J, st, st.band_localfreq[bd], st.band_polb[bd], j, P, D.scale, s_cf, buf + k * T);
+      const int bd = NB == 2 ? p : min(2 * p + k, J.nbands - 1);
+      put_entries<C>(J, st, st.band_localfreq[bd], st.band_polb[bd], j, P[NB == 2 ? k : 0], D.scale, s_cf, buf + k * T);
     }
   };
 
   const int b0 = blockIdx.x * G * blocks_per_group + g;
   fetch_param(b0, pbuf);
-  fetch_param(b0 + G, pbuf + 1);
+  fetch_param(b0 + G, pbuf + NB);
   cp_async_wait_all();
   __syncthreads();
   int tb = 0;
   bool staged = false;     // raw and tables hold the block the loop is at
 #pragma unroll 1
   for (int it = 0; it < blocks_per_group; it++) {
-    const int bi = b0 + it * G;
-    if (blockIdx.x * G * blocks_per_group + it * G >= nblk) break;   // no group of the CTA has a block left
-    const BlockParam &P = pbuf[it & 1], &Pn = pbuf[(it + 1) & 1];   // this block, the group's next one
+    const int u = b0 + it * G, bi = u * NB;   // the group's unit and its first block
+    if (blockIdx.x * G * blocks_per_group + it * G >= nunit) break;   // no group of the CTA has a unit left
+    const BlockParam *const P = pbuf + (it & 1) * NB, *const Pn = pbuf + ((it + 1) & 1) * NB;   // this unit, the group's next one
     if (!staged) {
       load_raw(P, 0);
       build_tables(P, 0, tabs + tb * SETS * T);
@@ -574,37 +666,63 @@ fstep_pair_kernel(const __grid_constant__ DevJob J, const DevStation *__restrict
     staged = false;
     // blocks that are not processed: zero spectra (all blocks of a warp, where it holds several groups)
     if (NT <= 32 ? !__any_sync(0xffffffffu, live) : !live) {
-      if (bi < nblk)
+      for (int b = bi; b < min(nblk, bi + NB); b++)
         for (int bd = 0; bd < J.nbands; bd++) {
-          float2 *row = spec + (((size_t)st.freq_index[st.band_localfreq[bd]] * nblk + bi) * J.ninputs + st.band_input[bd]) * N;
+          float2 *row = spec + (((size_t)st.freq_index[st.band_localfreq[bd]] * nblk + b) * J.ninputs + st.band_input[bd]) * N;
           for (int c = j; c < N; c += NT) row[c] = make_float2(0.f, 0.f);
         }
-      sync_group<NT, CTA>(g);   // all have read this block's parameters
-      fetch_param(bi + 2 * G, &pbuf[it & 1]);
+      sync_group<NT, CTA>(g);   // all have read this unit's parameters
+      fetch_param(u + 2 * G, pbuf + (it & 1) * NB);
       cp_async_wait_all();
       sync_group<NT, CTA>(g);
       continue;
     }
     const bool more = it < blocks_per_group - 1;
 #pragma unroll 1
-    for (int p = 0; p < D.npairs; p++) {
-      const int bd0 = 2 * p, bd1 = min(2 * p + 1, J.nbands - 1);
-      const bool has1 = 2 * p + 1 < J.nbands;
-      const int lf0 = st.band_localfreq[bd0], lf1 = SAME ? lf0 : st.band_localfreq[bd1];
+    for (int p = 0; p < D.nfields; p++) {
+      // A pair's second band is always there, but has1 stays a condition: without
+      // it the compiler runs the two bands' corrections and stores into one another
+      // (complex pairs of two frequencies, 16 stations, 1024 points: F-step
+      // 0.90 -> 0.96 ms).
+      const int bd0 = NB == 2 ? p : 2 * p, bd1 = NB == 2 ? p : min(2 * p + 1, J.nbands - 1);
+      const bool has1 = NB == 2 ? bi + 1 < nblk : 2 * p + 1 < J.nbands;
+      const int lf0 = st.band_localfreq[bd0], lf1 = SAME || NB == 2 ? lf0 : st.band_localfreq[bd1];
       const float2 *tab0 = tabs + tb * SETS * T, *tab1 = SAME ? tab0 : tab0 + T;
       sync_group<NT, CTA>(g);   // tables written; the previous pair's exchange buffer read
-      unsigned int vm0 = vmask, vm1 = vmask;
-      if (S.bandmask && bi < nblk && P.state != 0) {   // EDV4 masks blank frames per band
+      unsigned int vm0 = vmask, vm1 = NB == 2 ? vmask1 : vmask;
+      if (NB == 1 && S.bandmask && bi < nblk && P[0].state != 0) {   // EDV4 masks blank frames per band
         const unsigned long long *bm = S.bandmask + ((size_t)s * nblk + bi) * J.nbands;
         const unsigned long long m0 = bm[bd0], m1 = bm[bd1];
         if (m0 | m1) {
-          const int smp0 = P.nearestsample + jb;
+          const int smp0 = P[0].nearestsample + jb;
           int q = smp0 / fsamp, r = smp0 - q * fsamp;
-          q -= P.fr0;
+          q -= P[0].fr0;
 #pragma unroll 1
           for (int t = 0; t < 16; t++) {
             vm0 &= ~((unsigned int)((m0 >> min(q, 63)) & 1ull) << t);
             vm1 &= ~((unsigned int)((m1 >> min(q, 63)) & 1ull) << t);
+            r += NT;
+            while (r >= fsamp) {
+              r -= fsamp;
+              q++;
+            }
+          }
+        }
+      }
+      if (NB == 2 && S.bandmask) {
+#pragma unroll 1
+        for (int k = 0; k < NB; k++) {
+          const BlockParam &B = P[k];
+          if (bi + k >= nblk || B.state == 0) continue;
+          const unsigned long long m = S.bandmask[((size_t)s * nblk + bi + k) * J.nbands + p];
+          const int smp0 = B.nearestsample + jb;
+          int q = smp0 / fsamp, r = smp0 - q * fsamp;
+          q -= B.fr0;
+#pragma unroll 1
+          for (int t = 0; m && t < 16; t++) {
+            const unsigned int off = (unsigned int)((m >> min(q, 63)) & 1ull) << t;
+            if (k) vm1 &= ~off;
+            else vm0 &= ~off;
             r += NT;
             while (r >= fsamp) {
               r -= fsamp;
@@ -641,10 +759,36 @@ fstep_pair_kernel(const __grid_constant__ DevJob J, const DevStation *__restrict
             v[t].im = make_float2(w0.y * x.x, w1.y * x.y);
           }
         };
-        if (!fast) {
+        if constexpr (NB == 2) {
+          const int nb = J.nbits;
+          uint32_t wa[16], wb[16];
+          const int s0 = load_words(P[0], p * D.width, vm0, wa), s1 = load_words(P[1], p * D.width, vm1, wb);
+#pragma unroll
+          for (int t = 0; t < 16; t++) {
+            wa[t] >>= (s0 + t * NT * D.ts_bits) & 31;
+            wb[t] >>= (s1 + t * NT * D.ts_bits) & 31;
+          }
+          if (D.kind == 1) {
+            const float2 bias = dup(-8388736.0f);   // as below
+#pragma unroll
+            for (int t = 0; t < 16; t++) {
+              auto part = [&](unsigned int k) {
+                return r16::add2(make_float2(__uint_as_float(__byte_perm(wa[t], 0x4B000000u, 0x7650u + k)),
+                                             __uint_as_float(__byte_perm(wb[t], 0x4B000000u, 0x7650u + k))), bias);
+              };
+              rotate(t, part(0), CPLX ? part(1) : dup(0.f));
+            }
+          } else {
+            const uint32_t m = (1u << nb) - 1u;
+#pragma unroll
+            for (int t = 0; t < 16; t++)
+              rotate(t, make_float2(s_lut[wa[t] & m], s_lut[wb[t] & m]),
+                     CPLX ? make_float2(s_lut[(wa[t] >> nb) & m], s_lut[(wb[t] >> nb) & m]) : dup(0.f));
+          }
+        } else if (!fast) {
           // any layout: the fields' own bytes, read here; time samples narrower
           // than a byte start at a bit
-          const int smp0 = P.nearestsample + jb;
+          const int smp0 = P[0].nearestsample + jb;
           int q = smp0 / fsamp, r = smp0 - q * fsamp;
           const uint8_t *fr = data + (long long)q * fbytes + 32;
           const int nb = J.nbits, off = D.width * p, nbit = min(D.width, D.ts_bits - off);
@@ -676,7 +820,7 @@ fstep_pair_kernel(const __grid_constant__ DevJob J, const DevStation *__restrict
         } else if (D.kind == 1) {
           // code c as the float 2^23 + c (byte placed under the exponent 0x4B)
           const float2 bias = dup(-8388736.0f);
-              const unsigned int s0 = 0x7650u + (unsigned int)(sh >> 3);
+          const unsigned int s0 = 0x7650u + (unsigned int)(sh >> 3);
 #pragma unroll
           for (int t = 0; t < 16; t++) {
             auto byte = [&](unsigned int k) { return __uint_as_float(__byte_perm(raw[t], 0x4B000000u, s0 + k)); };
@@ -711,7 +855,7 @@ fstep_pair_kernel(const __grid_constant__ DevJob J, const DevStation *__restrict
       }
       if (PC) xb[pc_slot<C>(jb)] = make_float4(psr.x, psr.y, psi.x, psi.y);
       // the next column, or the next block's first one, while the transform runs
-      const bool last_pair = p == D.npairs - 1;
+      const bool last_pair = p == D.nfields - 1;
       if (last_pair ? more : (p + 1) % D.ppc == 0) load_raw(last_pair ? Pn : P, last_pair ? 0 : (p + 1) / D.ppc);
       const int lsb0 = st.lsb[lf0], lsb1 = SAME ? lsb0 : st.lsb[lf1];
       const float2 sg = make_float2(lsb0 ? -1.f : 1.f, lsb1 ? -1.f : 1.f);   // real data: which half of the bins
@@ -719,23 +863,47 @@ fstep_pair_kernel(const __grid_constant__ DevJob J, const DevStation *__restrict
       // phase-cal: bin of thread j < nbins, which collects threads j, j + nbins,
       // ... in that order; one thread per bin and block, blocks ordered by the
       // group's barriers, so the sums do not depend on timing
-      int pcbin = -1;
-      if (PC && pcout && j < pcn && P.state != 0)
-        pcbin = (int)((pcs0 + (unsigned long long)P.nearestsample + (unsigned long long)j) % (unsigned long long)pcn);
+      int pcbin = -1, pcm0 = NT, pcm1 = NT;   // two blocks: bin j, which collects threads pcm0 (pcm1), + nbins, ...
+      if (PC && pcout && j < pcn) {
+        const unsigned long long n = (unsigned long long)pcn;
+        if constexpr (NB == 2) {
+          auto first = [&](const BlockParam &B) {
+            return (int)(((unsigned long long)j + n - (pcs0 + (unsigned long long)B.nearestsample) % n) % n);
+          };
+          if (P[0].state != 0) pcm0 = first(P[0]);
+          if (P[1].state != 0) pcm1 = first(P[1]);
+          if (pcm0 < NT || pcm1 < NT) pcbin = j;
+        } else if (P[0].state != 0) {
+          pcbin = (int)((pcs0 + (unsigned long long)P[0].nearestsample + (unsigned long long)j) % n);
+        }
+      }
       auto pcal = [&]() {
         if (PC && pcbin >= 0) {
           float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-          for (int m = j; m < NT; m += pcn) {
-            const float4 q = xb[pc_slot<C>(m)];
-            a.x += q.x;
-            a.y += q.y;
-            a.z += q.z;
-            a.w += q.w;
-          }
           float2 *o = pcout + (size_t)bd0 * pf.maxbins + pcbin;
+          if constexpr (NB == 2) {
+            for (int m = pcm0; m < NT; m += pcn) {
+              const float4 q = xb[pc_slot<C>(m)];
+              a.x += q.x;
+              a.z += q.z;
+            }
+            for (int m = pcm1; m < NT; m += pcn) {
+              const float4 q = xb[pc_slot<C>(m)];
+              a.x += q.y;
+              a.z += q.w;
+            }
+          } else {
+            for (int m = j; m < NT; m += pcn) {
+              const float4 q = xb[pc_slot<C>(m)];
+              a.x += q.x;
+              a.y += q.y;
+              a.z += q.z;
+              a.w += q.w;
+            }
+          }
           atomicAdd(&o->x, a.x * D.scale);
           if (CPLX) atomicAdd(&o->y, a.z * D.scale);
-          if (has1) {
+          if (NB == 1) {
             o += pf.maxbins;
             atomicAdd(&o->x, a.y * D.scale);
             if (CPLX) atomicAdd(&o->y, a.w * D.scale);
@@ -852,7 +1020,8 @@ fstep_pair_kernel(const __grid_constant__ DevJob J, const DevStation *__restrict
           else J.paired ? both(0, true) : both(0, false);
         } else {
           auto one = [&](int lane, const float2 *tab, int bd, int lf, int lsb) {
-            float2 *row = spec + (((size_t)st.freq_index[lf] * nblk + bi) * J.ninputs + st.band_input[bd]) * N;
+            const int b = NB == 2 ? bi + lane : bi;
+            float2 *row = spec + (((size_t)st.freq_index[lf] * nblk + b) * J.ninputs + st.band_input[bd]) * N;
 #pragma unroll
             for (int t = 0; t < NOUT; t++) {
               bool conj;
@@ -870,9 +1039,9 @@ fstep_pair_kernel(const __grid_constant__ DevJob J, const DevStation *__restrict
       }
       if constexpr (C::TBUF == 1) sync_group<NT, CTA>(g);   // the tables are rewritten in place
       if (!last_pair || more) {
-        // every thread has read this block's parameters before the exchanges'
-        // synchronisation: the buffer takes those of the block after the next
-        if (last_pair) fetch_param(bi + 2 * G, &pbuf[it & 1]);
+        // every thread has read this unit's parameters before the exchanges'
+        // synchronisation: the buffer takes those of the unit after the next
+        if (last_pair) fetch_param(u + 2 * G, pbuf + (it & 1) * NB);
         tb ^= C::TBUF - 1;
         build_tables(last_pair ? Pn : P, last_pair ? 0 : p + 1, tabs + tb * SETS * T);
         if (last_pair) cp_async_wait_all();
@@ -882,25 +1051,30 @@ fstep_pair_kernel(const __grid_constant__ DevJob J, const DevStation *__restrict
   }
 }
 
-// Launches the kernel of a transform length and pair form for one data type.
-template <int CPLX, bool PC>
-cudaError_t launch(const DevJob &J, const DevStation *stations, const SubintArrays &S, int nblk, int items,
-                   const PairDecode &D, const BlockParam *bp, float2 *spec, const PcalFuse &pf, cudaStream_t st)
+#define GX_PAIR_ARGS                                                                                               \
+  const DevJob &J, const DevStation *stations, const SubintArrays &S, int nblk, int items, const PairDecode &D,   \
+      const BlockParam *bp, float2 *spec, const PcalFuse &pf, cudaStream_t st
+
+// Launches the kernel of a transform length for one data type; ONE: one band and
+// two blocks at a time, else the pairs.
+template <int CPLX, bool PC, bool ONE>
+cudaError_t launch(GX_PAIR_ARGS)
 {
   const bool same = J.pair_same != 0;
   auto go = [&](auto kernel, int groups, int cta, size_t sm) -> cudaError_t {
     cudaError_t e = smem_opt_in((const void *)kernel, sm);
     if (e != cudaSuccess) return e;
-    const dim3 grid((nblk + items * groups - 1) / (items * groups), J.nstations);
+    const int nunit = ONE ? (nblk + 1) / 2 : nblk;
+    const dim3 grid((nunit + items * groups - 1) / (items * groups), J.nstations);
     kernel<<<grid, cta, sm, st>>>(J, stations, S, bp, nblk, items, D, spec, pf);
     return cudaGetLastError();
   };
-#define GX_PAIR_CASE(FLV)                                                                            \
-  case FLV: {                                                                                        \
-    using C = Cfg<FLV, CPLX>;                                                                        \
-    return same ? go(fstep_pair_kernel<FLV, CPLX, true, PC>, C::G, C::CTA, smem_bytes<FLV, CPLX>(1)) \
-                : go(fstep_pair_kernel<FLV, CPLX, false, PC>, C::G, C::CTA, smem_bytes<FLV, CPLX>(2)); \
-  }
+#define GX_PAIR_FORM(FLV, LANES) \
+  go(fstep_pair_kernel<FLV, CPLX, LANES, PC>, Cfg<FLV, CPLX>::G, Cfg<FLV, CPLX>::CTA, smem_bytes<FLV, CPLX, LANES>())
+#define GX_PAIR_CASE(FLV)                                                                                  \
+  case FLV:                                                                                                \
+    if constexpr (ONE) return GX_PAIR_FORM(FLV, kTwoBlocks);                                               \
+    else return same ? GX_PAIR_FORM(FLV, kSameBands) : GX_PAIR_FORM(FLV, kTwoBands);
   switch (J.fftlen) {
     GX_PAIR_CASE(128)
     GX_PAIR_CASE(256)
@@ -911,17 +1085,18 @@ cudaError_t launch(const DevJob &J, const DevStation *stations, const SubintArra
     GX_PAIR_CASE(8192)
   }
 #undef GX_PAIR_CASE
+#undef GX_PAIR_FORM
   return cudaErrorNotSupported;
 }
 
-#define GX_PAIR_ARGS                                                                                               \
-  const DevJob &J, const DevStation *stations, const SubintArrays &S, int nblk, int items, const PairDecode &D,   \
-      const BlockParam *bp, float2 *spec, const PcalFuse &pf, cudaStream_t st
-// one translation unit each: the kernels of a data type, without and with phase-cal
+// one translation unit each: the kernels of a data type, and of one band at a
+// time, without and with phase-cal
 cudaError_t launch_real(GX_PAIR_ARGS);
 cudaError_t launch_cplx(GX_PAIR_ARGS);
 cudaError_t launch_real_pc(GX_PAIR_ARGS);
 cudaError_t launch_cplx_pc(GX_PAIR_ARGS);
+cudaError_t launch_one(GX_PAIR_ARGS);
+cudaError_t launch_one_pc(GX_PAIR_ARGS);
 
 }  // namespace pr
 }  // namespace gx

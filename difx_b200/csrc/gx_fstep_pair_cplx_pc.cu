@@ -6,7 +6,7 @@ namespace pr {
 
 cudaError_t launch_cplx_pc(GX_PAIR_ARGS)
 {
-  return launch<1, true>(J, stations, S, nblk, items, D, bp, spec, pf, st);
+  return launch<1, true, false>(J, stations, S, nblk, items, D, bp, spec, pf, st);
 }
 
 }  // namespace pr

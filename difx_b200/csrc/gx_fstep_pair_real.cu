@@ -6,7 +6,7 @@ namespace pr {
 
 cudaError_t launch_real(GX_PAIR_ARGS)
 {
-  return launch<0, false>(J, stations, S, nblk, items, D, bp, spec, pf, st);
+  return launch<0, false, false>(J, stations, S, nblk, items, D, bp, spec, pf, st);
 }
 
 }  // namespace pr

@@ -6,7 +6,7 @@ namespace pr {
 
 cudaError_t launch_real_pc(GX_PAIR_ARGS)
 {
-  return launch<0, true>(J, stations, S, nblk, items, D, bp, spec, pf, st);
+  return launch<0, true, false>(J, stations, S, nblk, items, D, bp, spec, pf, st);
 }
 
 }  // namespace pr
