@@ -973,22 +973,25 @@ static gx_status setup(gx_handle *h)
     // Both X-steps move their accumulators through HBM once per pass (the
     // tensor-core form 128 x 128 complex per channel, the FP32 form its upper
     // super-tiles) and every pass ends in a partly filled round of CTAs, so
-    // passes are long: up to 32768 blocks and 40 GB of spectra, at most 30% of
-    // the device memory free at open.  The tensor-core form stops at 4096: its
-    // tensor-memory sums run over a slice's whole share of the pass and the MMA
-    // truncates them, so their error grows with the run (24 dual-polarisation
-    // stations, 8 x 128 channels, one slice, split form against 64 bits, cross
-    // and autocorrelations: 512 blocks 2.8e-6 and 6.7e-6, 4096 blocks 2.1e-5 and
-    // 6.0e-5, 32768 blocks 1.7e-4 and 4.5e-4; F and X 11.87 ms a subint in passes of 4096,
-    // 11.30 in one of 32768).
-    size_t spec_budget = size_t(40) << 30;
+    // passes are long: up to 4096 blocks and 40 GB of spectra, at most 30% of
+    // the device memory free at open; up to 32768 blocks where that takes at
+    // most 1/32 of it, so that a program's later handles and buffers find room
+    // (4 stations of 128 channels, 25000 blocks, F-step in passes of 4096 and in
+    // one: 0.59 and 0.37 ms, spectra 0.13 and 0.82 GB).  The tensor-core form
+    // always stops at 4096: its tensor-memory sums run over a slice's whole share
+    // of the pass and the MMA truncates them, so their error grows with the run
+    // (24 dual-polarisation stations, 8 x 128 channels, one slice, split form
+    // against 64 bits, cross and autocorrelations: 512 blocks 2.8e-6 and 6.7e-6,
+    // 4096 blocks 2.1e-5 and 6.0e-5, 32768 blocks 1.7e-4 and 4.5e-4; F and X 11.87 ms a
+    // subint in passes of 4096, 11.30 in one of 32768).
+    size_t fr = size_t(128) << 30;   // a host-only handle plans for about one B200
     {
-      size_t fr = 0, tot = 0;
-      if (h->device >= 0 && cudaSetDevice(h->device) == cudaSuccess && cudaMemGetInfo(&fr, &tot) == cudaSuccess)
-        spec_budget = std::max(size_t(1) << 30, std::min(spec_budget, fr / 10 * 3));
+      size_t f = 0, tot = 0;
+      if (h->device >= 0 && cudaSetDevice(h->device) == cudaSuccess && cudaMemGetInfo(&f, &tot) == cudaSuccess) fr = f;
     }
-    const size_t longest = h->tc ? 4096 : 32768;
-    chunk = (int)std::min(longest, std::max<size_t>(64, spec_budget / per_block));
+    const size_t spec_budget = std::max(size_t(1) << 30, std::min(size_t(40) << 30, fr / 10 * 3));
+    const size_t usual = std::min<size_t>(4096, std::max<size_t>(64, spec_budget / per_block));
+    chunk = (int)(h->tc ? usual : std::max(usual, std::min<size_t>(32768, fr / 32 / per_block)));
   }
   if (chunk > J.blocks_per_send) chunk = J.blocks_per_send;
   chunk = std::max(1, chunk);
