@@ -164,7 +164,6 @@ static gx_status setup(gx_handle *h)
     return h->fail(GX_ERR_ARG, "DATA FRAME SIZE is not a whole number of time samples");
 
   DevJob &J = h->J;
-  J.deltapol_any = 0;
   J.nstations = d.nstations;
   J.nbands = s0.nbands;
   J.nbits = s0.nbits;
@@ -183,8 +182,6 @@ static gx_status setup(gx_handle *h)
   J.nfr = J.fftlen / J.stride;
   if (J.stride & (J.stride - 1)) return h->fail(GX_ERR_UNSUPPORTED, "array stride must be a power of two");
   J.fringe_order = d.fringe_rotation_order;
-  J.lgstride = 0;
-  while ((1 << J.lgstride) < J.stride) J.lgstride++;
   J.half = (cplx ? 2 * J.nfr : J.nfr) / 2;
   J.unpacksamples = cplx ? f0.nchan : 2 * f0.nchan;
   J.sampletime = 1.0 / (2.0 * f0.bw_mhz);
@@ -254,7 +251,6 @@ static gx_status setup(gx_handle *h)
       h->band_input[s][b] = D.band_input[b];
     }
     for (int b = 0; b < x.nbands; b++) D.band_polb[b] = (D.deltapol && x.band_pol[b] != 'R') ? 1 : 0;
-    if (D.deltapol) J.deltapol_any = 1;
     for (int b = 0; b + 1 < x.nbands; b += 2)
       if (D.band_localfreq[b] != D.band_localfreq[b + 1] || D.band_polb[b] != D.band_polb[b + 1]) J.pair_same = 0;
   }
@@ -1073,19 +1069,6 @@ static gx_status setup(gx_handle *h)
       for (int b = 0; b < 256; b++) lut[b] = (float)((b - off) / 3.3);
       J.lut_offset = off;
       J.lut_div = 3.3;
-      // The same levels without a table lookup: 1 / 3.3 as a two-float sum and
-      // one fused multiply-add, used only if it reproduces every entry.
-      const double bias = 8388608.0 + off;
-      const float hi = (float)(1.0 / 3.3), lo = (float)(1.0 / 3.3 - (double)hi);
-      bool ok = (double)(float)bias == bias;
-      for (int b = 0; ok && b < 256; b++) {
-        const float x = (float)(8388608.0 + b) - (float)bias;
-        ok = std::fma(x, hi, x * lo) == lut[b];
-      }
-      J.lut_affine = ok ? 1 : 0;
-      J.lut_bias = (float)bias;
-      J.lut_hi = hi;
-      J.lut_lo = lo;
     }
     // Tensor-core operands: a power-of-two scale that brings the spectrum of
     // noise with the r.m.s. level of the decode table to an r.m.s. near 8, so

@@ -49,11 +49,9 @@ struct DevJob {
   int nrows;              // rows in use of the fullest freq
   int nfreqs;
   int blocks_per_send;
-  int sb_items;           // paired-band F-step: FFT blocks per group and CTA (0: 4)
+  int sb_items;           // paired-band F-step: units of work per group and CTA (0: by the pass, pair_items)
   int flaglen;
-  int lgstride;           // log2(stride): FFT length, channels and stride are powers of two
   int fringe_order;       // FRINGE ROTN ORDER: 1 pre-F linear, 2 pre-F quadratic, 0 post-F (real data)
-  int deltapol_any;       // some station has a second (polarisation B) fractional-sample rotator
   int paired;             // spectra rows 2s and 2s + 1 interleaved by channel: [freq][block][row pair][channel][2]
   int pair_same;          // bands 2p and 2p + 1 share local freq and fractional-sample rotator at every station
   double sampletime;      // us
@@ -63,11 +61,6 @@ struct DevJob {
   float lut[256];         // level of each sample code (VDIF decode table), staged to shared memory
   int lut_zero;           // some code's level is zero
   double lut_offset, lut_div;   // 8-bit codes: level = (code - lut_offset) / lut_div
-  // 8-bit codes by arithmetic: level = fma(x, lut_hi, x * lut_lo) with
-  // x = float(2^23 + code) - lut_bias; set only when the host has checked that
-  // this equals lut[code] for all 256 codes (lut_affine = 1)
-  int lut_affine;
-  float lut_bias, lut_hi, lut_lo;
 };
 
 // Offset of (input row, channel c) inside the spectra of one (freq, block):

@@ -19,7 +19,7 @@ static PairDecode pair_decode(const DevJob &J)
   D.load = pairs && (words || narrow);
   D.ncol = !D.load ? D.nfields : words ? D.ts_bits / 32 : 1;
   D.ppc = D.nfields / D.ncol;
-  D.kind = (!J.cplx && J.nbits <= 2) ? 0 : (J.nbits == 8 && J.lut_affine) ? 1 : 2;
+  D.kind = (!J.cplx && J.nbits <= 2) ? 0 : (J.nbits == 8 && J.lut_offset == kCodeOffset) ? 1 : 2;
   D.scale = D.kind == 1 ? (float)(1.0 / J.lut_div) : 1.0f;
   return D;
 }

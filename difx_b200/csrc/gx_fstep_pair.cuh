@@ -71,9 +71,13 @@ struct PairDecode {
   int ts_bits;       // bits of a time sample
   int ncol, ppc;     // columns loaded per time sample, pairs per column
   int load;          // 1: pairs are read as aligned columns, 0: bytes of the field one by one
-  int kind;          // 0: level pair from a table of 1- or 2-bit real codes, 1: 8-bit codes, 2: level table
-  float scale;       // kind 1: level = (code - 128) scale, the scale carried by the rotator
+  // 0: level pair from a table of 1- or 2-bit real codes, 1: 8-bit codes by arithmetic, 2: level table
+  int kind;
+  float scale;       // kind 1: level = (code - kCodeOffset) scale, the scale carried by the rotator
 };
+
+// The offset of 8-bit codes that kind 1 takes off; symmetric ones (127.5) use the table.
+constexpr int kCodeOffset = 128;
 
 namespace pr {
 
@@ -769,7 +773,7 @@ fstep_pair_kernel(const __grid_constant__ DevJob J, const DevStation *__restrict
             wb[t] >>= (s1 + t * NT * D.ts_bits) & 31;
           }
           if (D.kind == 1) {
-            const float2 bias = dup(-8388736.0f);   // as below
+            const float2 bias = dup(-(float)(8388608 + kCodeOffset));   // as below
 #pragma unroll
             for (int t = 0; t < 16; t++) {
               auto part = [&](unsigned int k) {
@@ -793,7 +797,7 @@ fstep_pair_kernel(const __grid_constant__ DevJob J, const DevStation *__restrict
           const uint8_t *fr = data + (long long)q * fbytes + 32;
           const int nb = J.nbits, off = D.width * p, nbit = min(D.width, D.ts_bits - off);
           const uint32_t m = (1u << nb) - 1u;
-          auto level = [&](uint32_t c) { return D.kind == 1 ? (float)(int)(c & m) - 128.f : s_lut[c & m]; };
+          auto level = [&](uint32_t c) { return D.kind == 1 ? (float)(int)(c & m) - (float)kCodeOffset : s_lut[c & m]; };
 #pragma unroll
           for (int t = 0; t < 16; t++) {
             uint32_t f = 0;
@@ -819,7 +823,7 @@ fstep_pair_kernel(const __grid_constant__ DevJob J, const DevStation *__restrict
           for (int t = 0; t < 16; t++) rotate(t, s_pl[(raw[t] >> sh) & m], dup(0.f));
         } else if (D.kind == 1) {
           // code c as the float 2^23 + c (byte placed under the exponent 0x4B)
-          const float2 bias = dup(-8388736.0f);
+          const float2 bias = dup(-(float)(8388608 + kCodeOffset));
           const unsigned int s0 = 0x7650u + (unsigned int)(sh >> 3);
 #pragma unroll
           for (int t = 0; t < 16; t++) {

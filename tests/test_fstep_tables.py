@@ -1,15 +1,15 @@
-"""Host-side arithmetic of the station-block F-step's shared-memory tables.
+"""Host-side arithmetic of the paired-band F-step's shared-memory tables.
 
-The kernel (difx_b200/csrc/gx_fstep_sb.cu) takes the stride-256 radix-16
+The kernel (difx_b200/csrc/gx_fstep_pair.cuh) takes the stride-256 radix-16
 twiddles W_4096^(r m), m < 256, as the product of two 15 x 16 rows
 (B[r][m mod 16] = W_4096^(r (m mod 16)), A[r][m / 16] = W_256^(r (m / 16)))
-and decodes 8-bit VDIF codes (format_vdif.c: level = (b - 128) / 3.3) by
-fma(x, hi, x * lo) with 1/3.3 = hi + lo when the host finds that equal to the
-level table.  These tests restate both in numpy: the factorised twiddle stays
-within a few FP32 ulps of the exact one, and the two-term FMA reproduces every
-entry of the reference's table.  They also check the index arithmetic of the
-phase-cal sums the kernel forms: the exchange-buffer pad slots it parks them
-in, and the one bin a thread's samples share.
+and decodes 8-bit VDIF codes (format_vdif.c: level = (b - 128) / 3.3) as the
+exact integer b - 128, formed from the float 2^23 + b, with 1 / 3.3 carried by
+the rotator.  These tests restate both in numpy: the factorised twiddle stays
+within a few FP32 ulps of the exact one, and the integers times FP32(1 / 3.3)
+within two of the reference's table.  They also check the index arithmetic of
+the phase-cal sums the kernel forms: the exchange-buffer pad slots it parks
+them in, and the one bin a thread's samples share.
 """
 import numpy as np
 
@@ -54,29 +54,20 @@ def test_stride16_rows_are_the_table_section():
                 assert abs(_w(256, r * m) - _w(F, r * m * F // 256)) < 1e-12
 
 
-def _two_term_levels(off):
-    hi = np.float32(1.0 / 3.3)
-    lo = np.float32(1.0 / 3.3 - float(hi))
+def test_8bit_levels_by_arithmetic():
     b = np.arange(256)
-    x = (b - off).astype(np.float32)
-    xlo = (x * lo).astype(np.float32)
-    # fma(x, hi, xlo): x * hi is exact in float64 (8-bit x 24-bit), and the sum
-    # spans under 53 bits, so one rounding to FP32 is the fused result
-    return (x.astype(np.float64) * np.float64(hi) + xlo.astype(np.float64)).astype(np.float32)
-
-
-def test_8bit_levels_by_two_term_fma_match_table():
-    b = np.arange(256)
+    codes = (np.uint32(0x4B000000) | b.astype(np.uint32)).view(np.float32)   # the float 2^23 + b
+    np.testing.assert_array_equal(codes, (8388608.0 + b).astype(np.float32))
+    x = codes + np.float32(-8388736.0)
+    np.testing.assert_array_equal(x, (b - 128).astype(np.float32))           # exact
     table = ((b - 128.0) / 3.3).astype(np.float32)     # format_vdif.c lut8bit, FP64 then FP32
-    np.testing.assert_array_equal(_two_term_levels(128.0), table)
+    level = x * np.float32(1.0 / 3.3)
+    assert np.all(np.abs(level - table) <= 2 * np.spacing(np.abs(table)))    # a rounded factor, a rounded product
 
 
-def test_8bit_symmetric_offset_keeps_table():
-    # the kernel forms x as float(2^23 + b) - (2^23 + offset); with the 127.5
-    # offset that bias is not an FP32 value, so the host leaves the table on
-    bias = 8388608.0 + 127.5
-    assert float(np.float32(bias)) != bias
-    assert float(np.float32(8388608.0 + 128.0)) == 8388608.0 + 128.0
+def test_8bit_symmetric_offset_is_not_an_integer():
+    # so the symmetric levels, (b - 127.5) / 3.3, come from the table
+    assert float(np.float32(8388608.0 + 127.5)) != 8388608.0 + 127.5
 
 
 def test_phase_cal_pad_slots_are_free():
