@@ -1445,7 +1445,7 @@ gx_status gx_get_tiles(const gx_handle *h, int *xmac_variant, int *fstep_items)
 {
   if (!h) return GX_ERR_ARG;
   if (xmac_variant) *xmac_variant = h->xvar;
-  if (fstep_items) *fstep_items = h->J.sb_items > 0 ? h->J.sb_items : 4;
+  if (fstep_items) *fstep_items = h->J.sb_items;
   return GX_OK;
 }
 

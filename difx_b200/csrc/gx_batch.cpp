@@ -347,7 +347,7 @@ gx_status gx_batch_tune_tiles(gx_batch *b, const gx_subint_desc *const *subs, in
     const Key k{h->tc ? 1 : 0, h->tc ? 0 : h->xs.T, h->tc ? 0 : h->xs.ST, h->J.fftlen, h->J.nbits, h->J.cplx, h->J.nbands};
     classes[k].push_back((int)j);
   }
-  const int items[] = {2, 4, 8};
+  const int items[] = {0, 2, 4, 8};   // 0, the choice by the pass, first: the others must beat it
   for (auto &kv : classes) {
     const std::vector<int> &members = kv.second;
     int jb = members[0];
@@ -356,7 +356,7 @@ gx_status gx_batch_tune_tiles(gx_batch *b, const gx_subint_desc *const *subs, in
     gx_handle *h = b->jobs[jb];
     const int nxv = h->tc ? 1 : gx::kXmacVariants;
     double best = 1e30;
-    int bx = 0, bf = 4;
+    int bx = 0, bf = 0;
     for (int xv = 0; xv < nxv; xv++)
       for (int fi : items) {
         if ((r = gx_set_tiles(h, xv, fi)) != GX_OK) return b->fail(r, h->err);

@@ -558,7 +558,9 @@ gx_status gx_sta(const gx_handle *h, const float *results, int dump_channels, fl
 
 /* Launch shapes a tuner may choose per job; results do not depend on them.
    xmac_variant: the FP32 X-step's channel tile and stage depth (0 or 1);
-   fstep_items: FFT blocks a station-block F-step group takes per CTA (0: 4). */
+   fstep_items: FFT blocks (with an odd band count, pairs of them) that a group
+   of the paired-band F-step takes per CTA; 0, as a handle is opened: chosen per
+   pass from its length and the number of stations. */
 gx_status gx_set_tiles(gx_handle *h, int xmac_variant, int fstep_items);
 gx_status gx_get_tiles(const gx_handle *h, int *xmac_variant, int *fstep_items);
 

@@ -35,3 +35,14 @@ def test_batch_null_calls():
     assert L.gx_batch_info(None, None, None, None) == 1
     assert L.gx_batch_close(None) == 1
     assert L.gx_batch_last_error(None) == b"null batch"
+
+
+def test_launch_shapes_of_an_untuned_handle():
+    """0 blocks per group -- chosen per pass -- is what a handle starts with, reports and can be set back to."""
+    c = gxcorr.Correlator.from_desc(capi.job_desc_from_spec(jobs.spec_c1()), device=-1)
+    assert tuple(c.tiles()) == (0, 0)
+    c.set_tiles(1, 8)
+    assert tuple(c.tiles()) == (1, 8)
+    c.set_tiles(0, 0)
+    assert tuple(c.tiles()) == (0, 0)
+    c.close()
