@@ -40,6 +40,9 @@ __host__ __device__ constexpr int xmac_tiles()
 template <int TB, int ST, int CT, bool DIAG>
 __host__ __device__ constexpr int xmac_warps() { return xmac_tiles<TB, ST, DIAG>() / 2 * (CT / 16); }
 
+// Blocks that a product is summed over in one register, at most.
+__host__ __device__ constexpr int xmac_run(bool two) { return two ? 128 : 256; }
+
 // One CTA: super-tile pair blockIdx.x (DIAG: the pairs on the diagonal, else
 // those above it, row-major) of frequency f for CT channels from c0 =
 // blockIdx.y CT, over the blocks of K-split slice ks.  Stages -- KB blocks x ST
@@ -58,19 +61,20 @@ __host__ __device__ constexpr int xmac_warps() { return xmac_tiles<TB, ST, DIAG>
 // the shared-memory latency.  64 stations, 4096 channels, 125 blocks: 5.41 ->
 // 2.77 ms, 26 of the 36 T FMA lanes a second that 128 a clock are (16 stations,
 // 6250 blocks: 2.81 -> 1.18 ms, 28 of them).
-// The sums of a product stay short: after kRun blocks in one register, TWO
+// The sums of a product stay short: after a run of blocks in one register, TWO
 // register levels (where the shape leaves the registers) or the accumulators in
-// memory take them over, so the FP32 error does not grow with the pass.
+// memory take them over, so the FP32 error does not grow with the pass.  A slice
+// is cut into equal runs of at most xmac_run(TWO) blocks: runs of the longest
+// length and a rest cost the same and err more (16 stations, 5000 blocks in slices
+// of 320: 4.0e-7 of the 64-bit values in runs of 256 and 64, 3.6e-7 in two of 160).
 template <int TB, int ST, int CT, int KB, int NSTAGE, bool DIAG, int MINB, bool TWO>
 __global__ void __launch_bounds__(xmac_warps<TB, ST, CT, DIAG>() * 32, MINB)
 xmac_fp32_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int N, int nsuper, int ks_count,
-                 int kper, float2 *__restrict__ acc, int accumulate, int *__restrict__ err)
+                 int kper, int run_stages, float2 *__restrict__ acc, int accumulate, int *__restrict__ err)
 {
   constexpr int NCW = xmac_warps<TB, ST, CT, DIAG>();
   constexpr int NTILE = xmac_tiles<TB, ST, DIAG>();
   constexpr int STAGE = KB * ST * CT;   // float2 per stage per operand
-  constexpr int kRun = TWO ? 128 : 256;
-  static_assert(kRun % KB == 0, "runs of whole stages");
   static_assert(NTILE % 2 == 0 && CT % 16 == 0 && ST % kTA == 0 && kTA % TB == 0, "a warp takes two tiles by 16 channels");
   extern __shared__ __align__(128) float2 xsm[];
   float2 *sI = xsm;                     // [NSTAGE][KB][ST][CT]
@@ -176,7 +180,7 @@ xmac_fp32_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int N, 
   int st = 0;
 #pragma unroll 1
   do {
-    const int run = min(nstages, st + kRun / KB);
+    const int run = min(nstages, st + run_stages);
 #pragma unroll 1
     for (; st < run; st++) {
       const int buf = st % NSTAGE;
@@ -376,9 +380,11 @@ static cudaError_t launch_t(const float2 *spec, int nblk, int rows, int NI, int 
   // the variants add the same blocks into each slice
   static_assert(16 % KB == 0, "slice boundaries must be whole stages");
   const int kper = ((nblk + ks - 1) / ks + 15) / 16 * 16;
+  const int units = kper / 16, runs = (units * 16 + xmac_run(TWO) - 1) / xmac_run(TWO);
+  const int run_stages = (units + runs - 1) / runs * (16 / KB);
   // super-tile pairs fastest: the pairs that share a channel group's spectra run together
   dim3 grid(npairs, (N + CT - 1) / CT, nfreqs * ks);
-  kernel<<<grid, xmac_warps<TB, ST, CT, DIAG>() * 32, sm, st>>>(map, nblk, N, nsuper, ks, kper, acc, accumulate, err);
+  kernel<<<grid, xmac_warps<TB, ST, CT, DIAG>() * 32, sm, st>>>(map, nblk, N, nsuper, ks, kper, run_stages, acc, accumulate, err);
   return cudaGetLastError();
 }
 
