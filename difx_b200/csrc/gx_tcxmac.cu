@@ -302,7 +302,7 @@ xmac_tc_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int NP, i
     const uint32_t at0 = place(r, e0), at1 = place(r1, e1);
     for (int t = 0; t < nt; t++) {
       const int st = t % kStages, o = t % kOpStages;
-      const bool loaded = mbar_wait(smem_u32(full + st), (uint32_t)(t / kStages) & 1u) && !*s_abort;
+      const bool loaded = mbar_wait(smem_u32(full + st), (uint32_t)(t / kStages) & 1u);
       const int kv = min(kKT, nblk - (t0 + t) * kKT);
       const float4 *stg = reinterpret_cast<const float4 *>(staging + st * kStageBytes);
       // (value 0 re, im, value 1 re, im) at block k; of an odd piece of a pair, input r is the second

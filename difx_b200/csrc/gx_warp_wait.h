@@ -1,8 +1,7 @@
 // A stage that ends the same way for every lane of a warp.  A bounded wait can
-// succeed in one lane and run out in its neighbour, and a lane can read the
-// abort flag a moment before or after it is set; lanes that decided alone would
-// then part -- some at the warp's next barrier, some at the CTA's -- and wait
-// for one another without limit.  So a lane whose wait ran out still works
+// succeed in one lane and run out in its neighbour; lanes that decided alone
+// would then part -- some at the warp's next barrier, some at the CTA's -- and
+// wait for one another without limit.  So a lane whose wait ran out still works
 // through the stage (its sums are thrown away) and the lanes vote at the
 // barrier that ends it: all go on, or all leave.  (A vote in front of the work
 // instead put its latency on the stage's critical path: tensor-core X-step of 64
@@ -17,7 +16,9 @@
 
 namespace gx {
 
-// good: this lane's wait succeeded and it saw no abort; all: true in every lane
+// good: this lane's wait succeeded (a warp need not look for the CTA's abort flag
+// stage by stage: what it waits for then stops coming, and its own wait runs
+// out); all: true in every lane
 // if every lane's argument is; sync: the warp's barrier.
 template <class All, class Sync>
 GX_HOST_DEVICE bool warp_goes_on(bool good, All all, Sync sync)

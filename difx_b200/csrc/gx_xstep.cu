@@ -184,7 +184,7 @@ xmac_fp32_kernel(const __grid_constant__ CUtensorMap spec_map, int nblk, int N, 
 #pragma unroll 1
     for (; st < run; st++) {
       const int buf = st % NSTAGE;
-      const bool good = mbar_wait(smem_u32(full + buf), (uint32_t)(st / NSTAGE) & 1u) && !*s_abort;
+      const bool good = mbar_wait(smem_u32(full + buf), (uint32_t)(st / NSTAGE) & 1u);
       const float2 *bi_ = sI + buf * STAGE + ti * kTA * CT + c;
       const float2 *bj_ = sJ + buf * STAGE + tj * TB * CT + c;
 #pragma unroll 1
