@@ -90,6 +90,35 @@ int gx_bl_localfreq(const gx_baseline_desc &b, int f)
 
 static int bl_localfreq(const gx_baseline_desc &b, int f) { return gx_bl_localfreq(b, f); }
 
+// K-split slices of the FP32 X-step: enough CTAs for at least two per SM, in
+// whole waves of 148 SMs where possible, and at least 64 blocks a slice.  Up to
+// 16 slices (64 of 8 inputs, whose accumulators are small), and where those
+// leave SMs idle -- few channels of few freqs -- up to 64 of at least 128 blocks
+// (1 x 64 channels, X stage with 16 slices and with 64: 16 inputs, 40000 blocks
+// 0.70 -> 0.21 ms; 64 inputs, 20000 blocks 1.36 -> 0.56).
+static int xmac_slices(const XmacShape &xs, int nchan, int nfreqs, int chunk)
+{
+  auto tiles = [&](int ct) { return (long long)((nchan + ct - 1) / ct) * nfreqs; };
+  long long base = tiles(xs.CT) * xs.npairs;
+  int kmax = xs.ST == 8 ? 64 : 16;
+  // more than one super-tile: a launch for the diagonal (32 channels a CTA), one for the others
+  const long long few = xs.nsuper > 1 ? std::min(tiles(32) * xs.nsuper, tiles(xs.CT) * (xs.npairs - xs.nsuper)) : base;
+  if (few * 16 < 296 && chunk >= 128 * 16) {
+    base = few;
+    kmax = std::min(64, chunk / 128);
+  }
+  kmax = std::max(1, std::min(kmax, chunk / 64));
+  int best = 1;
+  double best_score = -1;
+  for (int ks = 1; ks <= kmax; ks++) {
+    const long long ctas = base * ks;
+    const double waves = std::ceil(ctas / 148.0);
+    const double score = ctas / (waves * 148.0) * std::min(1.0, ctas / 296.0);
+    if (score > best_score + 1e-9) { best_score = score; best = ks; }
+  }
+  return best;
+}
+
 static gx_status setup(gx_handle *h)
 {
   const gx_job_desc &d = h->jd;
@@ -1014,35 +1043,13 @@ static gx_status setup(gx_handle *h)
     while (best < kmax && base * best < 2 * 148) best++;
     h->ks = best;
   } else {
-    long long base = (long long)((J.nchan + xs.CT - 1) / xs.CT) * xs.npairs * h->nfmain;
-    // K-split: enough CTAs for at least two per SM, rounded to whole waves of
-    // 148 SMs where possible, keeping at least 64 blocks per slice
-    // (up to 64 slices of 8 inputs, whose accumulators are small)
-    const int kmax = std::max(1, std::min(xs.ST == 8 ? 64 : 16, chunk / 64));
-    int best = 1;
-    double best_score = -1;
-    for (int ks = 1; ks <= kmax; ks++) {
-      const long long ctas = base * ks;
-      const double waves = std::ceil(ctas / 148.0);
-      const double eff = ctas / (waves * 148.0);
-      const double score = eff * std::min(1.0, ctas / 296.0);
-      if (score > best_score + 1e-9) { best_score = score; best = ks; }
-    }
-    h->ks = best;
+    h->ks = xmac_slices(xs, J.nchan, h->nfmain, chunk);
   }
   // zoom X-step K-split: as the FP32 X-step's, over the zoom freqs
   h->zks = 1;
   if (!h->zfreq.empty()) {
     const XmacShape &zx = h->zxs;
-    const long long base = (long long)((h->nzchan + zx.CT - 1) / zx.CT) * zx.npairs * (long long)h->zfreq.size();
-    const int kmax = std::max(1, std::min(16, chunk / 64));
-    double best_score = -1;
-    for (int ks = 1; ks <= kmax; ks++) {
-      const long long ctas = base * ks;
-      const double waves = std::ceil(ctas / 148.0);
-      const double score = ctas / (waves * 148.0) * std::min(1.0, ctas / 296.0);
-      if (score > best_score + 1e-9) { best_score = score; h->zks = ks; }
-    }
+    h->zks = xmac_slices(zx, h->nzchan, (int)h->zfreq.size(), chunk);
     h->zacc_slice = h->zfreq.size() * (size_t)zx.npairs * zx.ST * zx.ST * h->nzchan;
   }
   // F-step concurrency: FFT slots per CTA of the slot-per-band kernel

@@ -320,14 +320,28 @@ __global__ void finalise_vis_kernel(const ProdEntry *__restrict__ prods, int npr
   // 64-station 4096-channel job was slower (0.46 -> 0.55 ms): it keeps the form below.
   if (N <= (int)blockDim.x) {
     if (c0 >= N) return;
-    float2 t = a[0];
-#pragma unroll 8
-    for (int k = 1; k < ks_count; k++) {
+    // four sums of every fourth slice, then those: with up to 64 slices one sum
+    // after the other would err more than the slices themselves (11 stations of
+    // 64 channels, 37 slices: 1.3e-7 of the 64-bit values, 1.0e-7 in four)
+    float2 p[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) p[i] = make_float2(0.f, 0.f);
+    int k = 0;
+#pragma unroll 2
+    for (; k + 4 <= ks_count; k += 4)
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const float2 v = a[(size_t)(k + i) * ks_stride];
+        p[i].x += v.x;
+        p[i].y += v.y;
+      }
+    for (; k < ks_count; k++) {
       const float2 v = a[(size_t)k * ks_stride];
-      t.x += v.x;
-      t.y += v.y;
+      p[0].x += v.x;
+      p[0].y += v.y;
     }
-    out[0] = make_float2(t.x, pe.conj ? -t.y : t.y);
+    const float re = (p[0].x + p[1].x) + (p[2].x + p[3].x), im = (p[0].y + p[1].y) + (p[2].y + p[3].y);
+    out[0] = make_float2(re, pe.conj ? -im : im);
     return;
   }
   float2 s[4];

@@ -1,7 +1,7 @@
 """Long sums of the FP32 X-step: slices of several runs, whose sums pass from the
 registers they grow in to a second level (8 and 16 rows: registers, 32 rows: the
 accumulators in memory), block counts off the runs and the stages, one and
-several passes, and the largest K-split of 8 rows.
+several passes, and the largest K-split, as few channels get it.
 
 One band of 64 channels keeps the oracle quick.  Tolerance as the parity tests':
 records within 1e-5; the two launch shapes add the same blocks in the same order
@@ -21,10 +21,10 @@ pytestmark = pytest.mark.gpu
     (2, 4997, 0),        # 8 rows: 64 slices of 80 blocks
     (2, 9001, 0),        # 64 slices of two runs
     (3, 9000, 4500),     # in two passes
-    (9, 5003, 0),        # 16 rows: 16 slices of 320 in three runs
-    (9, 5003, 2501),     # two runs, two passes
-    (17, 9001, 0),       # 32 rows: 16 slices of 576 in three runs
-    (17, 10007, 5003),   # two runs, two passes
+    (9, 9001, 0),        # 16 rows: 64 slices of two runs
+    (9, 5003, 1999),     # 16 slices of a run, three passes
+    (17, 17409, 0),      # 32 rows: 64 slices of two runs
+    (17, 6001, 3000),    # 23 slices, two passes
     (33, 5003, 0),       # off the diagonal too
 ])
 def test_long_slices(stations, blocks, chunk, oracle_lib):
