@@ -8,7 +8,7 @@
 // issue slots, FMA pipe and shared memory run out before HBM does.  Packing the
 // two bands of a pair into f32x2 registers halves the instructions of the
 // butterflies and the exchange-address work and, where the bands are the two
-// polarisations of one frequency, shares the rotator tables and products: 60
+// polarisations of one frequency, shares the rotator tables and products: 65
 // thread instructions a band sample against 82 of one band at a time.  64 data
 // registers a thread leave 16 warps an SM, so what is left is latency (issue
 // active 45-60 %, FMA pipe 42-54 %).  F-step times against the kernels it

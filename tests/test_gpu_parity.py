@@ -57,7 +57,7 @@ CASES = {
     "cplx8": lambda: (jobs.spec_cplx8(), dict()),
     "cplx8_invalid": lambda: (jobs.spec_cplx8(name="cx8bad", seed=23), dict(invalid_frac=0.08)),
     "c2small": lambda: (jobs.spec_c2small(), dict(invalid_frac=0.01)),
-    # long transforms (register-resident radix-16 F-step)
+    # long transforms
     "cplx8_4096": lambda: (jobs.spec_long("cx8l", 8, "COMPLEX", "U", 4096, 41), dict(invalid_frac=0.03)),
     "cplx8_4096_lsb": lambda: (jobs.spec_long("cx8ll", 8, "COMPLEX", "L", 4096, 43), dict(invalid_frac=0.03)),
     "real2_8192": lambda: (jobs.spec_long("r2x", 2, "REAL", "U", 4096, 47), dict(invalid_frac=0.03)),
@@ -393,7 +393,7 @@ PCAL_CASES = {
     "cplx2_pcal": lambda: (jobs.spec_long("cx2pc", 2, "COMPLEX", "U", 128, 87, pcal_interval_mhz=1),
                            dict(invalid_frac=0.03)),
     # the C3 sample format (8 complex 8-bit bands, 16-byte time samples) with
-    # 4096-point transforms: the station-block F-step forms the bin sums
+    # 4096-point transforms: the paired-band F-step forms the bin sums
     # (16 bins divide its 256 threads per transform); real4_pcal takes that
     # path with four transform groups per CTA (32 bins, 64 threads)
     "cplx8_4096_pcal": lambda: (jobs.spec_long("cx8pcl", 8, "COMPLEX", "U", 4096, 91, pcal_interval_mhz=1,
