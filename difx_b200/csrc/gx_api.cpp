@@ -91,24 +91,37 @@ int gx_bl_localfreq(const gx_baseline_desc &b, int f)
 static int bl_localfreq(const gx_baseline_desc &b, int f) { return gx_bl_localfreq(b, f); }
 
 // K-split slices of the FP32 X-step: enough CTAs for at least two per SM, in
-// whole waves of 148 SMs where possible, and at least 64 blocks a slice.  Up to
-// 16 slices (64 of 8 inputs, whose accumulators are small), and where those
-// leave SMs idle -- few channels of few freqs -- up to 64 of at least 128 blocks
-// (1 x 64 channels, X stage with 16 slices and with 64: 16 inputs, 40000 blocks
-// 0.70 -> 0.21 ms; 64 inputs, 20000 blocks 1.36 -> 0.56).
+// whole waves of 148 SMs where possible, at least 64 blocks a slice and at most 16
+// slices (64 of 8 inputs, whose accumulators are small).  Where 16 leave SMs idle
+// -- few channels of few freqs -- the number up to 64 with the least time by the
+// waves of each launch, a CTA an SM, and the accumulators' way to memory and
+// back.  1 x 64 channels, X stage with 16 slices and with the chosen ones: 16
+// inputs, 40000 blocks 0.70 -> 0.21 ms; 64 inputs, 20000 blocks 1.36 -> 0.48.
 static int xmac_slices(const XmacShape &xs, int nchan, int nfreqs, int chunk)
 {
   auto tiles = [&](int ct) { return (long long)((nchan + ct - 1) / ct) * nfreqs; };
-  long long base = tiles(xs.CT) * xs.npairs;
-  int kmax = xs.ST == 8 ? 64 : 16;
   // more than one super-tile: a launch for the diagonal (32 channels a CTA), one for the others
-  const long long few = xs.nsuper > 1 ? std::min(tiles(32) * xs.nsuper, tiles(xs.CT) * (xs.npairs - xs.nsuper)) : base;
-  if (few * 16 < 296 && chunk >= 128 * 16) {
-    base = few;
-    kmax = std::min(64, chunk / 128);
-  }
-  kmax = std::max(1, std::min(kmax, chunk / 64));
+  const bool two = xs.nsuper > 1;
+  const long long diag = two ? tiles(32) * xs.nsuper : tiles(xs.CT), off = two ? tiles(xs.CT) * (xs.npairs - xs.nsuper) : 0;
   int best = 1;
+  if (xs.ST > 8 && (two ? std::min(diag, off) : diag) * 16 < 296) {
+    const double mac = 1.0 / 45.0;   // ns of an SM per complex multiply-add: 128 lanes at three quarters
+    const double diag_block = (two || xs.ST == 32 ? 20 * 32 * 32 : 6 * 32 * 64) * mac, off_block = 16 * 64 * 16 * mac;
+    const double slice = 2.0 * sizeof(float2) * xs.npairs * xs.ST * xs.ST * nchan * nfreqs / 4000.0;   // ns, written and read at 4 TB/s
+    double least = 1e30;
+    for (int ks = 1; ks <= std::max(1, std::min(64, chunk / 64)); ks++) {
+      const int kper = ((chunk + ks - 1) / ks + 15) / 16 * 16;
+      const long long used = (chunk + kper - 1) / kper;   // slices that have blocks
+      const double t = ((double)((diag * used + 147) / 148) * diag_block + (double)((off * used + 147) / 148) * off_block) * kper + slice * ks;
+      if (t < least * 0.999) {
+        least = t;
+        best = ks;
+      }
+    }
+    return best;
+  }
+  const long long base = tiles(xs.CT) * xs.npairs;
+  const int kmax = std::max(1, std::min(xs.ST == 8 ? 64 : 16, chunk / 64));
   double best_score = -1;
   for (int ks = 1; ks <= kmax; ks++) {
     const long long ctas = base * ks;

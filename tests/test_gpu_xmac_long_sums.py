@@ -22,9 +22,9 @@ pytestmark = pytest.mark.gpu
     (2, 9001, 0),        # 64 slices of two runs
     (3, 9000, 4500),     # in two passes
     (9, 9001, 0),        # 16 rows: 64 slices of two runs
-    (9, 5003, 1999),     # 16 slices of a run, three passes
+    (9, 5003, 1999),     # three passes
     (17, 17409, 0),      # 32 rows: 64 slices of two runs
-    (17, 6001, 3000),    # 23 slices, two passes
+    (17, 6001, 3000),    # two passes
     (33, 5003, 0),       # off the diagonal too
 ])
 def test_long_slices(stations, blocks, chunk, oracle_lib):
