@@ -90,6 +90,26 @@ int gx_bl_localfreq(const gx_baseline_desc &b, int f)
 
 static int bl_localfreq(const gx_baseline_desc &b, int f) { return gx_bl_localfreq(b, f); }
 
+// K-split slices of the tensor-core X-step over passes of `chunk` blocks.  One CTA
+// per SM (all 512 tensor-memory columns); every slice adds a full accumulator
+// write and finalise read, so the K dimension is split only while the grid is
+// under two waves of 148 SMs (at least 4 K-tiles per slice), and so that a slice
+// of a longer pass is no longer than one of kTcRun blocks': its sums stay in
+// tensor memory for the whole slice and the MMA truncates them, so their error
+// grows with it (24 dual-polarisation stations, 8 x 128 channels, one slice, split
+// form against 64 bits, cross and autocorrelations: 512 blocks 2.8e-6 and 6.7e-6,
+// 4096 blocks 2.1e-5 and 6.0e-5, 32768 blocks 1.7e-4 and 4.5e-4; F and X of the
+// 32768 blocks in passes of 4096 11.9 ms, in one slice 11.3, in eight 10.5).
+constexpr int kTcRun = 4096;
+static int tc_slices(int nchan, int nfreqs, int chunk)
+{
+  const long long base = (long long)(nchan / 2) * nfreqs;
+  const int kmax = std::max(1, std::min(16, std::min(chunk, kTcRun) / 64));
+  int ks = 1;
+  while (ks < kmax && base * ks < 2 * 148) ks++;
+  return chunk <= kTcRun ? ks : std::min(64, (int)(((long long)ks * chunk + kTcRun - 1) / kTcRun));
+}
+
 // K-split slices of the FP32 X-step: enough CTAs for at least two per SM, in
 // whole waves of 148 SMs where possible, at least 64 blocks a slice and at most 16
 // slices (64 of 8 inputs, whose accumulators are small).  Where 16 leave SMs idle
@@ -1015,13 +1035,9 @@ static gx_status setup(gx_handle *h)
     // the device memory free at open; up to 32768 blocks where that takes at
     // most 1/32 of it, so that a program's later handles and buffers find room
     // (4 stations of 128 channels, 25000 blocks, F-step in passes of 4096 and in
-    // one: 0.59 and 0.37 ms, spectra 0.13 and 0.82 GB).  The tensor-core form
-    // always stops at 4096: its tensor-memory sums run over a slice's whole share
-    // of the pass and the MMA truncates them, so their error grows with the run
-    // (24 dual-polarisation stations, 8 x 128 channels, one slice, split form
-    // against 64 bits, cross and autocorrelations: 512 blocks 2.8e-6 and 6.7e-6,
-    // 4096 blocks 2.1e-5 and 6.0e-5, 32768 blocks 1.7e-4 and 4.5e-4; F and X 11.87 ms a
-    // subint in passes of 4096, 11.30 in one of 32768).
+    // one: 0.59 and 0.37 ms, spectra 0.13 and 0.82 GB).  The tensor-core form only
+    // where slices of the same length as 4096-block passes have, and their
+    // accumulators, take no more (tc_slices).
     size_t fr = size_t(128) << 30;   // a host-only handle plans for about one B200
     {
       size_t f = 0, tot = 0;
@@ -1029,7 +1045,12 @@ static gx_status setup(gx_handle *h)
     }
     const size_t spec_budget = std::max(size_t(1) << 30, std::min(size_t(40) << 30, fr / 10 * 3));
     const size_t usual = std::min<size_t>(4096, std::max<size_t>(64, spec_budget / per_block));
-    chunk = (int)(h->tc ? usual : std::max(usual, std::min<size_t>(32768, fr / 32 / per_block)));
+    size_t longest = std::min<size_t>(32768, fr / 32 / per_block);
+    if (h->tc) {
+      const size_t slice = sizeof(float2) * (size_t)h->nfmain * J.nchan * kTcInputs * kTcInputs;
+      longest = std::min(longest, kTcRun * (std::min<size_t>(64, fr / 32 / slice) / tc_slices(J.nchan, h->nfmain, kTcRun)));
+    }
+    chunk = (int)std::max(usual, longest);
   }
   if (chunk > J.blocks_per_send) chunk = J.blocks_per_send;
   chunk = std::max(1, chunk);
@@ -1046,15 +1067,7 @@ static gx_status setup(gx_handle *h)
   }
   h->chunk = chunk;
   if (h->tc) {
-    // One CTA per SM (all 512 tensor-memory columns).  Every K-split slice
-    // adds a full accumulator write and finalise read, so the K dimension is
-    // split only while the grid is under two waves of 148 SMs (at least 4
-    // K-tiles per slice).
-    const long long base = (long long)(J.nchan / 2) * h->nfmain;
-    const int kmax = std::max(1, std::min(16, chunk / 64));
-    int best = 1;
-    while (best < kmax && base * best < 2 * 148) best++;
-    h->ks = best;
+    h->ks = tc_slices(J.nchan, h->nfmain, chunk);
   } else {
     h->ks = xmac_slices(xs, J.nchan, h->nfmain, chunk);
   }

@@ -145,14 +145,14 @@ typedef struct gx_job_desc {
   int write_autocorrs;     /* WRITE AUTOCORRS (also enables cross-pol autocorrelations) */
   int64_t max_data_bytes;  /* largest per-station data buffer one subint will pass */
   int xstep;               /* gx_xstep */
-  int block_chunk;         /* FFT blocks per device pass, 0 = automatic.  The tensor-core X-step sums a
-                              pass (or its K-split slice) in the MMA's FP32 accumulator, which truncates:
-                              its error grows with the pass */
+  int block_chunk;         /* FFT blocks per device pass, 0 = automatic.  The tensor-core X-step sums up to
+                              4096 blocks of a pass in the MMA's FP32 accumulator, which truncates: shorter
+                              passes err less */
   int64_t spectra_budget_bytes; /* with block_chunk 0: > 0 caps the spectra buffer and makes passes only as
                                    long as keeps accumulator traffic under a quarter of the spectra
                                    traffic (for many resident jobs); 0 = passes of up to 4096 blocks and
-                                   40 GB of spectra, at most 30% of the device memory free at open;
-                                   FP32 X-step: up to 32768 blocks within 1/32 of it */
+                                   40 GB of spectra, at most 30% of the device memory free at open, or
+                                   up to 32768 blocks within 1/32 of it */
 } gx_job_desc;
 
 /* One subint: the contents of one Core processslot (core.h:76-98). */

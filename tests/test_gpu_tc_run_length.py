@@ -1,6 +1,7 @@
 """How long a sum of the tensor-core X-step stays in tensor memory.  The MMA
 truncates its FP32 accumulator, so a long run loses a part of every sum that
-grows with the run; passes are limited to 4096 blocks for that reason.
+grows with the run; a pass of more than 4096 blocks is cut into slices for that
+reason.
 
 Tolerance of the autocorrelations (sums that grow evenly, so that every loss has
 one sign): each of the 6 MMAs that a 16-block step of the split form adds into a
@@ -23,17 +24,9 @@ def _spec():
                    nbits=2, subint_ns=BLOCKS * 8000, execute_seconds=2, max_delay_us=50.0, seed=77)
 
 
-@pytest.mark.parametrize("form", [capi.GX_XSTEP_TC_FP16_HILO, capi.GX_XSTEP_TC_FP16])
-def test_pass_length(form):
-    from difx_b200 import gxcorr
-    c = gxcorr.Correlator.from_desc(capi.job_desc_from_spec(_spec(), xstep=form), device=-1)
-    assert c.info.blocks_per_send == BLOCKS
-    assert c.info.block_chunk <= LONGEST
-    c.close()
-
-
 @pytest.mark.gpu
-def test_long_subint_autocorrelations():
+@pytest.mark.parametrize("chunk", [0, BLOCKS, 10923])   # by the handle, one pass, three
+def test_long_subint_autocorrelations(chunk):
     from difx_b200 import gxcorr
     spec = _spec()
     t0 = 100_000_000
@@ -45,7 +38,8 @@ def test_long_subint_autocorrelations():
     sd = capi.subint_desc_host(si, jobs.interpolators(jobs.write_job(spec, jobs._TMP + "/tcrun")["input"], spec, si, "host"))
     got = []
     for form in (capi.GX_XSTEP_TC_FP16_HILO, capi.GX_XSTEP_FP32):
-        c = gxcorr.Correlator.from_desc(capi.job_desc_from_spec(spec, xstep=form))
+        c = gxcorr.Correlator.from_desc(capi.job_desc_from_spec(spec, xstep=form, block_chunk=chunk))
+        assert c.info.blocks_per_send == BLOCKS
         got.append(c.subint(sd).copy())
         rl, bl, bw, ac, acw = c.offsets()
         c.close()
