@@ -1033,7 +1033,7 @@ static gx_status setup(gx_handle *h)
     // super-tiles) and every pass ends in a partly filled round of CTAs, so
     // passes are long: up to 4096 blocks and 40 GB of spectra, at most 30% of
     // the device memory free at open; up to 32768 blocks where that takes at
-    // most 1/32 of it, so that a program's later handles and buffers find room
+    // most 1/8 of it, so that a program's later handles and buffers find room
     // (4 stations of 128 channels, 25000 blocks, F-step in passes of 4096 and in
     // one: 0.59 and 0.37 ms, spectra 0.13 and 0.82 GB).  The tensor-core form only
     // where slices of the same length as 4096-block passes have, and their
@@ -1045,10 +1045,10 @@ static gx_status setup(gx_handle *h)
     }
     const size_t spec_budget = std::max(size_t(1) << 30, std::min(size_t(40) << 30, fr / 10 * 3));
     const size_t usual = std::min<size_t>(4096, std::max<size_t>(64, spec_budget / per_block));
-    size_t longest = std::min<size_t>(32768, fr / 32 / per_block);
+    size_t longest = std::min<size_t>(32768, fr / 8 / per_block);
     if (h->tc) {
       const size_t slice = sizeof(float2) * (size_t)h->nfmain * J.nchan * kTcInputs * kTcInputs;
-      longest = std::min(longest, kTcRun * (std::min<size_t>(64, fr / 32 / slice) / tc_slices(J.nchan, h->nfmain, kTcRun)));
+      longest = std::min(longest, kTcRun * (std::min<size_t>(64, fr / 8 / slice) / tc_slices(J.nchan, h->nfmain, kTcRun)));
     }
     chunk = (int)std::max(usual, longest);
   }

@@ -152,7 +152,7 @@ typedef struct gx_job_desc {
                                    long as keeps accumulator traffic under a quarter of the spectra
                                    traffic (for many resident jobs); 0 = passes of up to 4096 blocks and
                                    40 GB of spectra, at most 30% of the device memory free at open, or
-                                   up to 32768 blocks within 1/32 of it */
+                                   up to 32768 blocks within 1/8 of it */
 } gx_job_desc;
 
 /* One subint: the contents of one Core processslot (core.h:76-98). */

@@ -17,10 +17,10 @@ def _job(stations, subbands, nchan, blocks):
 def test_long_passes_leave_room():
     import torch
     from difx_b200 import gxcorr
-    # 32 inputs x 8 x 256 channels: 0.5 MB of spectra a block
-    per_block = 32 * 8 * 256 * 8
+    # 32 inputs x 16 x 256 channels: 1 MB of spectra a block, 34 GB in passes of 32768
+    per_block = 32 * 16 * 256 * 8
     free, _ = torch.cuda.mem_get_info()
-    c = gxcorr.Correlator.from_desc(capi.job_desc_from_spec(_job(16, 8, 256, 32768)))
+    c = gxcorr.Correlator.from_desc(capi.job_desc_from_spec(_job(16, 16, 256, 32768)))
     assert c.info.blocks_per_send == 32768
-    assert c.info.block_chunk <= max(4096, free // 32 // per_block)
+    assert c.info.block_chunk <= max(4096, free // 8 // per_block)
     c.close()
