@@ -1035,9 +1035,9 @@ static gx_status setup(gx_handle *h)
     // the device memory free at open; up to 32768 blocks where that takes at
     // most 1/8 of it, so that a program's later handles and buffers find room
     // (4 stations of 128 channels, 25000 blocks, F-step in passes of 4096 and in
-    // one: 0.59 and 0.37 ms, spectra 0.13 and 0.82 GB).  The tensor-core form only
-    // where slices of the same length as 4096-block passes have, and their
-    // accumulators, take no more (tc_slices).
+    // one: 0.59 and 0.37 ms, spectra 0.13 and 0.82 GB).  The tensor-core form cuts
+    // its longer passes into slices (tc_slices), whose accumulators take at most
+    // 1/8 too.
     size_t fr = size_t(128) << 30;   // a host-only handle plans for about one B200
     {
       size_t f = 0, tot = 0;
