@@ -41,7 +41,7 @@ template <int TB, int ST, int CT, bool DIAG>
 __host__ __device__ constexpr int xmac_warps() { return xmac_tiles<TB, ST, DIAG>() / 2 * (CT / 16); }
 
 // Blocks that a product is summed over in one register, at most.
-__host__ __device__ constexpr int xmac_run(bool two) { return two ? 128 : 256; }
+__host__ __device__ constexpr int xmac_run(bool two) { return two ? 96 : 256; }
 
 // One CTA: super-tile pair blockIdx.x (DIAG: the pairs on the diagonal, else
 // those above it, row-major) of frequency f for CT channels from c0 =
